@@ -220,6 +220,64 @@ def test_hyena_ops_backward_vs_oracle(io, bs, l, g, dg, hl):
         check(f"hyena_ops backward {io} {name} vs oracle", rel_l2(a, b), tol * (2.5 if name == "dC" else 1.0))
 
 
+@pytest.mark.parametrize("bs,l,g,dg,hl,views", [
+    (1, 1, 1, 16, 128, False), (1, 127, 2, 16, 7, False), (2, 128, 2, 16, 128, True), (3, 129, 3, 32, 127, False),
+    (5, 300, 2, 48, 1, True), (1, 257, 4, 16, 4, False), (2, 1000, 10, 16, 33, True), (1, 520, 310, 16, 128, False)])
+def test_backward_tensor_core_exact_on_integers(bs, l, g, dg, hl, views):
+    """The tensor-core backward at the edges of its chunks, segments, items and filters: small integers, whose products
+    and sums are exact in every format on the way, so all four gradients must be equal to the last bit (dz stays within
+    bf16's 256 because at most 64 taps are non-zero; dh is compared in fp32)."""
+    from vortex_b200 import ops
+
+    gen = torch.Generator().manual_seed(5)
+    D = g * dg
+    ri = lambda lo, hi, *sh: torch.randint(lo, hi + 1, sh, generator=gen).to(torch.bfloat16)  # noqa: E731
+    dy, x, Bm, Cm = (ri(-2, 2, bs, l, D), ri(-1, 1, bs, l, D), ri(-1, 1, bs, l, D), ri(-1, 1, bs, l, D))
+    y2 = ri(-3, 3, bs, l, D)
+    h = ri(-1, 1, g, hl)
+    if hl > 64:
+        h[:, 32:hl - 32] = 0
+    def dev(t):
+        if not views:
+            return t.cuda()
+        big = torch.full((bs + 1, l + 3, D + 24), float("nan"), dtype=t.dtype, device="cuda")
+        big[1:, 2:l + 2, 8:D + 8] = t.cuda()
+        return big[1:, 2:l + 2, 8:D + 8]
+    dx, dB, dC, dh = (t.cpu().double() for t in ops.gcg_bwd(dev(dy), dev(x), dev(Bm), dev(Cm), dev(y2), h.cuda()))
+    f = lambda t: t.double()  # noqa: E731
+    g2, z, w = f(dy) * f(Cm), f(x) * f(Bm), f(h).flip(1).repeat_interleave(dg, 0)       # w[d, lag]
+    dz = torch.zeros(bs, l, D, dtype=torch.double)
+    dw = torch.zeros(D, hl, dtype=torch.double)
+    for j in range(min(hl, l)):
+        dz[:, :l - j] += w[:, j] * g2[:, j:]
+        dw[:, j] = (g2[:, j:] * z[:, :l - j]).sum((0, 1))
+    assert dz.abs().max() <= 256
+    assert torch.equal(dx, dz * f(Bm)) and torch.equal(dB, dz * f(x)) and torch.equal(dC, f(dy) * f(y2))
+    assert torch.equal(dh, dw.view(g, dg, hl).sum(1).flip(1))
+
+
+@pytest.mark.parametrize("bs,l,g,dg,hl", [(1, 1, 1, 16, 4), (2, 127, 3, 16, 128), (3, 129, 2, 32, 7), (1, 1000, 20, 16, 33)])
+def test_training_forward_saves_the_filter_output(bs, l, g, dg, hl):
+    """The training forward's one launch against its definition, bit for bit: y2 = xcorr(h, B * x) rounded, y = C * y2
+    rounded, for gates of any magnitude (infinities and NaN included: the gate crosses the kernel unconverted)."""
+    from vortex_b200 import hyena_ops, ops
+
+    gen = torch.Generator().manual_seed(9)
+    x, Bm, Cm = (torch.randn(bs, l, g, dg, generator=gen).bfloat16() for _ in range(3))
+    Cm = (Cm.float() * torch.exp(20 * torch.randn(bs, l, g, dg, generator=gen))).bfloat16()
+    Cm.view(-1)[::97] = float("inf")
+    Cm.view(-1)[5::89] = float("nan")
+    h = (torch.randn(g, 1, hl, generator=gen) / hl ** 0.5).bfloat16()
+    x, Bm, Cm, h = (t.cuda() for t in (x, Bm, Cm, h))
+    y2 = hyena_ops.gcg_fwd(x, Bm, torch.ones_like(Cm), h)
+    y, got = ops.gcg_cl_fwd(*(t.view(bs, l, g * dg) for t in (Cm, Bm, x)), h, want_y2=True)
+    assert torch.equal(got.view_as(y2), y2)
+    want = Cm * y2
+    assert torch.equal(want.isnan(), y.view_as(y2).isnan()) and torch.equal(want.nan_to_num(7.), y.view_as(y2).nan_to_num(7.))
+    out = hyena_ops.two_pass_chunked_gate_conv_gate(x.requires_grad_(), Bm, Cm, h)
+    assert out.requires_grad and torch.equal(out.detach().nan_to_num(7.), want.nan_to_num(7.))
+
+
 # ------------------------------------------------------------------ seeded parity against the oracle
 def _engine_block(eng, p, D, G, K, layout, ip=None, heads=1):
     """The reference's two-call sequence (model.py:233-291) on the drop-in engine."""

@@ -141,6 +141,7 @@ SYMBOLS = {
     "vtx_featurizer_fwd": (C.c_int, [C.POINTER(FeaturizerParams), _p]),
     "vtx_gcg_fwd": (C.c_int, [C.POINTER(GcgParams), _p]),
     "vtx_gcg_cl_fwd": (C.c_int, [C.POINTER(GcgClParams), _p]),
+    "vtx_gcg_cl_fwd_saving": (C.c_int, [C.POINTER(GcgClParams), _p, _p]),
     "vtx_gcg_bwd": (C.c_int, [C.POINTER(GcgBwdParams), _p]),
     "vtx_fused_fir_fwd": (C.c_int, [C.POINTER(FusedFirParams), _p]),
     "vtx_modal_filter": (C.c_int, [C.POINTER(ModalParams), _p, _i, _p]),

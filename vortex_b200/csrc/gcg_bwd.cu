@@ -9,7 +9,8 @@
 //   dz[t]   = sum_j w[j] g2[t + j]                      (the same filter, run against time)
 //   dx      = dz * B,   dB = dz * x
 //   dw[j]   = sum over batch, time and the group's channels of g2[t] z[t - j]
-// Two kernels on the fp32 pipe (fp32 accumulation, one rounding on the way out):
+// bf16 operands with filters shared by multiples of 16 channels run on the tensor cores (gcg_bwd_tc.cu); every other call on
+// the two kernels here, on the fp32 pipe (fp32 accumulation, one rounding on the way out):
 //   data    a block owns 128 outputs of 32 channels; g2 with its K-1 rows of look-ahead sits in shared memory, a thread
 //           owns 16 consecutive samples of one channel and walks the taps 16 at a time with its window in registers
 //           (256 FMAs per 47 shared loads);
@@ -248,6 +249,11 @@ __global__ void __launch_bounds__(256) gcg_bwd_filter_kernel(vtx_gcg_bwd_params 
 }
 
 }  // namespace gbw
+
+namespace gbt {   // gcg_bwd_tc.cu: both reductions on the tensor cores
+bool takes(const vtx_gcg_bwd_params* p);
+int launch(const vtx_gcg_bwd_params* p, cudaStream_t stream);
+}  // namespace gbt
 }  // namespace vtx
 
 extern "C" int vtx_gcg_bwd(const vtx_gcg_bwd_params* p, void* stream) {
@@ -278,6 +284,7 @@ extern "C" int vtx_gcg_bwd(const vtx_gcg_bwd_params* p, void* stream) {
     const bool vec = p->D % nv == 0 && al(p->dy, p->dy_stride_b, p->dy_stride_l) && al(p->x, p->x_stride_b, p->x_stride_l) &&
                      al(p->Bg, p->b_stride_b, p->b_stride_l) && al(p->C, p->c_stride_b, p->c_stride_l) &&
                      al(p->y2, p->y2_stride_b, p->y2_stride_l) && al(p->dC, p->L * p->D, p->D);
+    if (vec && gbt::takes(p)) return gbt::launch(p, s);
     VTX_DISPATCH_IO(p->io_dtype, T, {
         const int ti = p->io_dtype == VTX_F32 ? 0 : p->io_dtype == VTX_BF16 ? 1 : 2;
         if (dev < 0 || dev >= 64 || !attr_set[dev][ti]) {

@@ -191,10 +191,10 @@ def gcg_cl_ok(q, k, v, h, bias_mode=BIAS_NONE) -> bool:
     return True
 
 
-def gcg_cl_fwd(q, k, v, h, bias=None, *, taps=TAPS_XCORR, bias_mode=BIAS_NONE, want_state=False):
+def gcg_cl_fwd(q, k, v, h, bias=None, *, taps=TAPS_XCORR, bias_mode=BIAS_NONE, want_state=False, want_y2=False):
     """Gate -> grouped FIR -> gate on channel-last operands q, k, v [B, L, D] (the hyena_ops layout with the group
     axes merged): one launch of the tensor-core kernel.  Returns y [B, L, D] and the inner cache [B, D, min(L, K-1)]
-    or None."""
+    or None -- with ``want_y2`` the filter output before the gate [B, L, D] in the cache's place."""
     _need_cuda(q, k, v, h, bias)
     B, L, D = q.shape
     h = _param(h, q)
@@ -212,6 +212,10 @@ def gcg_cl_fwd(q, k, v, h, bias=None, *, taps=TAPS_XCORR, bias_mode=BIAS_NONE, w
         state=_ptr(state) if (state is not None and ns > 0) else None, B=B, L=L, D=D, G=G, K=K, taps=taps,
         bias_mode=bias_mode if bias is not None else BIAS_NONE, io_dtype=_code(q))
     with _on(q):
+        if want_y2:
+            y2 = torch.empty_like(y)
+            _lib.check(_lib.lib().vtx_gcg_cl_fwd_saving(C.byref(p), _ptr(y2), _stream(q)))
+            return y, y2
         _lib.check(_lib.lib().vtx_gcg_cl_fwd(C.byref(p), _stream(q)))
     return y, state
 
