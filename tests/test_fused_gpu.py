@@ -646,6 +646,28 @@ def test_launch_count_follows_the_kernels_a_call_launches():
 
 
 @pytest.mark.gpu
+def test_prefill_caches_of_walks_with_several_items():
+    """The inner caches of a call whose CTAs walk several items each, the last chunks of the sequences among the first of
+    them: every cached product of every sequence, in calls repeated on the same input (a slot handed to the front end
+    before the cache warp has read it shows as samples of a later chunk)."""
+    from vortex_b200 import hyena_ops
+
+    B, L, D, K = 4, 1801, 4096, 128
+    g = torch.Generator(device="cuda").manual_seed(3)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    u, w3 = r(B, L, 3 * D).bfloat16(), (r(3 * D, 1, 3) / 3 ** 0.5).bfloat16()
+    h, Dp = (r(D // 16, 1, K) / K ** 0.5).bfloat16(), r(D).bfloat16()
+    tail = u[:, L - K - 1:].float()                        # the K - 1 cached samples and two rows before them
+    w = w3.float()[:, 0]
+    z = tail[:, :-2] * w[:, 0] + tail[:, 1:-1] * w[:, 1] + tail[:, 2:] * w[:, 2]
+    want = (z[..., 1::3] * z[..., 2::3]).transpose(1, 2)
+    for _ in range(4):
+        _, _, st = hyena_ops.hyena_mr_fwd(u, w3, None, h, Dp, want_state=True)
+        # one rounding to fp16's 11 bits, one to bf16's 8: 1.7e-3 relative L2; one stray chunk in a sequence is 1e-1
+        check("inner cache of a segmented prefill", rel_l2(st, want), 2e-3)
+
+
+@pytest.mark.gpu
 def test_fused_mr_call_cut_into_launches():
     """A call large enough to be cut into several launches (24 sequences of 8192 tokens, 4096 channels: 6.4 GB moved)
     gives, bit for bit, what single-launch calls on slices of the batch give, caches included; the oracle agrees on a

@@ -417,7 +417,10 @@ __global__ void __launch_bounds__(THREADS, 1) fused_mr_kernel(const __grid_const
                 yrow[s] = a.y + st.b * a.y_stride_b + (st.ts + r) * a.y_stride_l + (int64_t)g * CH;
                 nleft[s] = st.active ? (int)(st.te - st.ts) - r : 0;
             }
-            if (lane == 0) mbar_arrive(slot_free(cc & 1));      // the item's halo chunk has no epilogue
+            // The item's halo chunk has no epilogue, but its arrival must not count for the chunk before it in the slot, which
+            // the cache warp may still be reading: once the halo's tile is full, that chunk's slot has been freed by all.
+            if (!mbar_wait(kv_full(cc & 1), (cc >> 1) & 1u, 19)) { ok = false; break; }
+            if (lane == 0) mbar_arrive(slot_free(cc & 1));
             ++cc;
             for (int k = 1; k < nchunk; ++k, ++cc, ++oc) {
                 const int slot = cc & 1, dbuf = oc & 1;

@@ -266,7 +266,10 @@ gcg_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ C
                 x0[s] = (int)st.ts; bi[s] = (int)st.b; act[s] = st.active;
             }
             const int64_t d0 = (int64_t)blk * CH;
-            if (lane == 0) mbar_arrive(kv_free(cc % NSLOT));       // the item's halo chunk has no epilogue
+            // The item's halo chunk has no epilogue, but its arrival must not count for the chunk before it in the slot, which
+            // another epilogue warp may still be reading: once the halo's tile is full, that chunk has been freed by all.
+            if (!mbar_wait(kv_full(cc % NSLOT), (cc / NSLOT) & 1u, 44)) { ok = false; break; }
+            if (lane == 0) mbar_arrive(kv_free(cc % NSLOT));
             ++cc;
             for (int k = 1; k < nchunk; ++k, ++cc, ++oc) {
                 const int slot = cc % NSLOT, dbuf = oc & 1, qs = oc % NQ;
