@@ -101,6 +101,9 @@ typedef struct vtx_featurizer_params {
     int64_t io_dtype;
 } vtx_featurizer_params;
 int vtx_featurizer_fwd(const vtx_featurizer_params* p, void* stream);
+/* The same with z rows z_pitch >= L elements apart, z[b,c,t] at (b * C + c) * z_pitch + t (what lies between is not
+ * written): rows that start on 16-byte boundaries keep this kernel and the ones that read z on their fast paths. */
+int vtx_featurizer_fwd_pitched(const vtx_featurizer_params* p, int64_t z_pitch, void* stream);
 
 /* ------------------------------------------------------------------------
  * Gate -> grouped causal FIR -> gate, channel-first.  Any K >= 1, fp32 math

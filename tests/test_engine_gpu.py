@@ -426,6 +426,73 @@ def test_long_conv_segmented_and_complex(eng):
     check("test_engine_gpu.py:324 st2, O.modal_state(kv2, np.repeat(to_np(p['log_poles'])[..., 0], D // G, axis=0))", rel_l2(st2, O.modal_state(kv2, np.repeat(to_np(p["log_poles"])[..., 0], D // G, axis=0))), 1e-4)
 
 
+@pytest.mark.parametrize("io,B,L,D,G,S,cplx,layout,heads", [
+    ("bf16", 1, 1, 33, 33, 16, False, "split", 1),            # one sample; a warp with one lane past its 32 channels
+    ("f32", 2, 31, 31, 31, 16, False, "split", 1),            # less than a tile
+    ("bf16", 1, 63, 48, 3, 5, False, "interleaved", 1),       # shorter system, shared; one segment of two tiles
+    ("f16", 1, 64, 32, 32, 16, True, "split", 1),             # exactly one segment of two tiles
+    ("bf16", 2, 129, 40, 40, 16, False, "split", 1),          # two segments and one sample
+    ("f32", 1, 1001, 64, 64, 16, True, "split", 1),
+    ("bf16", 1, 4001, 96, 96, 16, False, "column_split", 3),  # many segments, ragged last one
+])
+def test_long_conv_tiles(io, B, L, D, G, S, cplx, layout, heads):
+    """The channel-first long convolution at the edges of its tiles, warps and segments against the mirrored oracle, on
+    rows that start on 16-byte boundaries and on rows that do not: same arithmetic, identical bits."""
+    from vortex_b200 import ops
+
+    p = make_block(31, B, L, D, G, 0, io, modal=True, S=S, complex_poles=cplx)
+    z = torch.randn(B, 3 * D, L, generator=torch.Generator().manual_seed(4)).to(DT[io])
+    rep = lambda a: np.repeat(a, D // G, axis=0)  # noqa: E731
+    lp = to_np(p["log_poles"])
+    if cplx:
+        poles, res = np.exp(lp[..., 0]) * np.exp(1j * to_np(p["theta"])), to_np(p["residues"]) + 1j * to_np(p["res_im"])
+        h = rep(O.modal_filter_complex(poles, res, L))
+    else:
+        h = rep(O.modal_filter(lp, to_np(p["residues"]), L))
+    ref, kv = O.long_conv_gate(to_np(z), h, to_np(p["Dp"]), D, io=io, layout=layout, num_heads=heads)
+    pc = cuda(p)
+    kw = dict(theta=pc["theta"], res_im=pc["res_im"]) if cplx else {}
+    kw.update(layout=layout, num_heads=heads)
+    pitch = (L + 15) // 16 * 16
+    outs = []
+    for shift in (0, 1):                                      # rows on and off the 16-byte boundaries
+        buf = torch.full((B, 3 * D, pitch + 2 * shift + 1 - (not shift)), float("nan"), dtype=DT[io], device="cuda")
+        zz = buf[..., shift:shift + L]
+        zz.copy_(z)
+        y, st = ops.iir_fwd(zz, pc["log_poles"], pc["residues"], pc["Dp"], D, **kw)
+        outs.append((y, st))
+    y, st = outs[0]
+    # mirrored: the rounding points are the oracle's; a sum in another order flips a last place here and there
+    check(f"long convolution tiles {io} L={L} y", rel_l2(y.permute(0, 2, 1), ref), TOL[io])
+    if cplx:
+        st_ref = O.modal_state_complex(kv, rep(poles))
+        check("long convolution tiles state", rel_l2(st, np.stack([st_ref.real, st_ref.imag], -1)), 2e-5)
+    else:
+        check("long convolution tiles state", rel_l2(st, O.modal_state(kv, rep(lp[..., 0]))), 2e-5)
+    assert torch.equal(y, outs[1][0]) and torch.equal(st, outs[1][1])
+
+
+@pytest.mark.parametrize("io,L,kind", [("bf16", 4001, "mr"), ("bf16", 129, "se"), ("f16", 1003, "se"), ("bf16", 127, "mr")])
+def test_rows_of_an_odd_length(eng, io, L, kind):
+    """The drop-in calls on lengths whose rows need padding to start on 16-byte boundaries: identical to the same calls on
+    a contiguous copy (which take the element-wise kernels), caches included."""
+    B, D, G, K = 2, 96, 6, 128 if kind == "mr" else 7
+    p = cuda(make_block(17, B, L, D, G, K, io))
+    dims = (D, 1, D, 16, G)
+    z, fs = eng.parallel_fir(F.conv1d, p["u"], p["w3"], None, L, dims=dims, gate=False, inference_params=True)
+    assert z.shape == (B, 3 * D, L) and z.stride(1) % 8 == 0
+    ref, fs_ref = O.featurizer(to_np(p["u"]), to_np(p["w3"]), io=io)
+    check(f"featurizer {io} L={L}", rel_l2(z, ref), 1e-4)
+    assert np.array_equal(to_np(fs), fs_ref.astype(np.float32))
+    kw = dict(dims=dims, groups=G, gated_bias=kind == "mr", dim_last=False, fir_length=K, gate=True, inference_params=True)
+    h = p["h"].repeat_interleave(D // G, 0)
+    y, st = eng.parallel_fir(F.conv1d, z, h, p["Dp"], L, **kw)
+    y2, st2 = eng.parallel_fir(F.conv1d, z.contiguous(), h, p["Dp"], L, **kw)
+    assert y.shape == (B, D, L) and torch.equal(st, st2)
+    # the two kernels sum the taps in different orders before one rounding of the filter output
+    check(f"gate-conv-gate {kind} {io} L={L}", rel_l2(y, y2), TOL[io])
+
+
 def test_padding_mask_and_errors(eng):
     B, L, D, G, K = 2, 40, 32, 2, 7
     p = cuda(make_block(21, B, L, D, G, K, "f32"))

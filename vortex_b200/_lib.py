@@ -139,6 +139,7 @@ SYMBOLS = {
     "vtx_debug_set_flag_poll_limit": (C.c_int, [_i]),
     "vtx_launch_count": (C.c_int64, []),
     "vtx_featurizer_fwd": (C.c_int, [C.POINTER(FeaturizerParams), _p]),
+    "vtx_featurizer_fwd_pitched": (C.c_int, [C.POINTER(FeaturizerParams), C.c_int64, _p]),
     "vtx_gcg_fwd": (C.c_int, [C.POINTER(GcgParams), _p]),
     "vtx_gcg_cl_fwd": (C.c_int, [C.POINTER(GcgClParams), _p]),
     "vtx_gcg_cl_fwd_saving": (C.c_int, [C.POINTER(GcgClParams), _p, _p]),

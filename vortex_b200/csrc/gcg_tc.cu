@@ -478,7 +478,7 @@ bool gcg_tc_shape(const vtx_gcg_params* p) {
         p->bias_mode == VTX_BIAS_ADD)
         return false;
     if (p->D % CH || p->G <= 0 || p->D % p->G || (p->D / p->G) % CH || p->head_dim % CH) return false;
-    if (p->y_stride_l != 1 || p->L % 8 || reinterpret_cast<uintptr_t>(p->y) % 16 || p->y_stride_d <= 0 || p->y_stride_d % 8 ||
+    if (p->y_stride_l != 1 || reinterpret_cast<uintptr_t>(p->y) % 16 || p->y_stride_d <= 0 || p->y_stride_d % 8 ||
         (p->B > 1 && (p->y_stride_b <= 0 || p->y_stride_b % 8)))
         return false;
     const void* ptrs[3] = {p->q, p->k, p->v};

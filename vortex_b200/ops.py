@@ -76,15 +76,31 @@ def launch_count() -> int:
     return int(_lib.lib().vtx_launch_count())
 
 
+def _rows(B: int, R: int, L: int, like: torch.Tensor, aligned: bool = True) -> torch.Tensor:
+    """Uninitialised [B, R, L] with every row on a 16-byte boundary: the first L samples of rows of whole 16-byte vectors
+    (a contiguous tensor where L is a multiple of them, or where ``aligned`` is false)."""
+    n = 16 // like.element_size()
+    pitch = -(-L // n) * n if aligned else L
+    t = torch.empty(B, R, pitch, device=like.device, dtype=like.dtype)
+    return t if pitch == L else t[..., :L]
+
+
+def _rows_aligned(t: torch.Tensor, *strides: int) -> bool:
+    return t.data_ptr() % 16 == 0 and all(s * t.element_size() % 16 == 0 for s in strides)
+
+
 # ----------------------------------------------------------------------------------------------
 def featurizer_fwd(u_blc: torch.Tensor, w: torch.Tensor, bias=None, mask=None, want_state=True):
-    """u_blc: logical [B, L, C] (any strides).  Returns z [B, C, L] and state [B, C, min(L,K-1)] or None."""
+    """u_blc: logical [B, L, C] (any strides).  Returns z [B, C, L] and state [B, C, min(L,K-1)] or None.
+
+    Rows of z start on 16-byte boundaries, so z is a slice of a padded tensor when L is not a multiple of 16 bytes (as
+    the reference's fp32 z is a slice of the padded convolution, engine.py:197-204)."""
     _need_cuda(u_blc, w, bias, mask)
     B, L, Cc = u_blc.shape
     w = _param(w, u_blc).reshape(Cc, -1)
     K = w.shape[1]
     bias, mask = _param(bias, u_blc), _param(mask, u_blc)
-    z = torch.empty(B, Cc, L, device=u_blc.device, dtype=u_blc.dtype)
+    z = _rows(B, Cc, L, u_blc)
     ns = min(L, K - 1)
     state = torch.empty(B, Cc, ns, device=u_blc.device, dtype=u_blc.dtype) if want_state else None
     p = _lib.FeaturizerParams(
@@ -93,7 +109,7 @@ def featurizer_fwd(u_blc: torch.Tensor, w: torch.Tensor, bias=None, mask=None, w
         mask=_ptr(mask), mask_dtype=_code(mask) if mask is not None else 0, z=_ptr(z),
         state=_ptr(state) if (state is not None and ns > 0) else None, B=B, L=L, C=Cc, K=K, io_dtype=_code(u_blc))
     with _on(u_blc):
-        _lib.check(_lib.lib().vtx_featurizer_fwd(C.byref(p), _stream(u_blc)))
+        _lib.check(_lib.lib().vtx_featurizer_fwd_pitched(C.byref(p), z.stride(1), _stream(u_blc)))
     return z, state
 
 
@@ -146,8 +162,9 @@ def _gcg_raw(q, k, v, sb, sh, sd, hd, h, bias, B, L, D, *, taps, bias_mode, mask
         y = torch.empty(B, L, D, device=dev, dtype=dt)
         ysb, ysd, ysl = L * D, 1, D
     else:
-        y = torch.empty(B, D, L, device=dev, dtype=dt)
-        ysb, ysd, ysl = D * L, L, 1
+        # operands with 16-byte aligned rows: the outputs' rows are laid out alike
+        y = _rows(B, D, L, q, all(_rows_aligned(t, s) for t, s in zip((q, k, v), sd if isinstance(sd, tuple) else (sd,) * 3)))
+        ysb, ysd, ysl = y.stride(0), y.stride(1), 1
     ns = min(L, K - 1)
     state = torch.empty(B, D, ns, device=dev, dtype=dt) if want_state else None
     sbs = sb if isinstance(sb, tuple) else (sb, sb, sb)
@@ -497,7 +514,7 @@ def causal_conv1d_varlen_states(x: torch.Tensor, cu_seqlens: torch.Tensor, state
 
 def iir_fwd(z_pre: torch.Tensor, log_poles, residues, bias, D: int, *, layout="split", num_heads=1, flip=False,
             theta=None, res_im=None, want_state=True, round_kv=True):
-    """Gate -> modal long convolution -> gate.  z_pre [B, 3D, L] -> y [B, D, L] (contiguous), state fp32
+    """Gate -> modal long convolution -> gate.  z_pre [B, 3D, L] -> y [B, D, L] (rows aligned as z_pre's are), state fp32
     [B, D, S] (or [B, D, S, 2] for complex poles) or None."""
     _need_cuda(z_pre, residues, bias)
     if z_pre.stride(2) != 1:
@@ -509,7 +526,7 @@ def iir_fwd(z_pre: torch.Tensor, log_poles, residues, bias, D: int, *, layout="s
     m, keep = _modal(log_poles, residues, z_pre, theta, res_im)
     cplx = theta is not None
     bias = _param(bias, z_pre)
-    y = torch.empty(B, D, L, device=z_pre.device, dtype=z_pre.dtype)
+    y = _rows(B, D, L, z_pre, _rows_aligned(z_pre, z_pre.stride(1)))
     state = None
     if want_state:
         state = torch.empty((B, D, m.S, 2) if cplx else (B, D, m.S), device=z_pre.device, dtype=torch.float32)
@@ -520,7 +537,7 @@ def iir_fwd(z_pre: torch.Tensor, log_poles, residues, bias, D: int, *, layout="s
         k=_ptr(k), k_stride_b=z_pre.stride(0), k_stride_h=sh, k_stride_d=sd,
         v=_ptr(v), v_stride_b=z_pre.stride(0), v_stride_h=sh, v_stride_d=sd, head_dim=hd, modal=m,
         bias=_ptr(bias), bias_dtype=_code(bias) if bias is not None else 0,
-        y=_ptr(y), y_stride_b=D * L, y_stride_d=L, y_stride_l=1, state=_ptr(state), scratch=_ptr(scratch),
+        y=_ptr(y), y_stride_b=y.stride(0), y_stride_d=y.stride(1), y_stride_l=1, state=_ptr(state), scratch=_ptr(scratch),
         B=B, L=L, D=D, round_kv=int(round_kv), io_dtype=_code(z_pre))
     with _on(z_pre):
         _lib.check(_lib.lib().vtx_iir_fwd(C.byref(p), _stream(z_pre)))
