@@ -9,6 +9,7 @@ import os
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG, "lib", "libvortex_b200.so")
+HOST_PATH = os.path.join(PKG, "lib", "_vtx_host.so")
 
 F32, BF16, F16 = 0, 1, 2
 QKV_SPLIT, QKV_INTERLEAVED, QKV_COLUMN_SPLIT = 0, 1, 2
@@ -161,6 +162,7 @@ SYMBOLS = {
     "vtx_decode_layer": (C.c_int, [C.POINTER(DecodeLayerParams), _p]),
 }
 
+_host = None
 _ERRORS = {-1: ValueError, -2: NotImplementedError, -3: ValueError, -4: RuntimeError, -5: RuntimeError}
 _lib = None
 
@@ -187,6 +189,29 @@ def lib() -> C.CDLL:
                                    f"ctypes {C.sizeof(st)}")
         _lib = handle
     return _lib
+
+
+def host():
+    """The native host module (``csrc/host.cpp``), bound to the loaded library.  Raises if it has not been built."""
+    global _host
+    if _host is None:
+        import importlib.util
+
+        import torch  # noqa: F401  (the module links against the libraries this loads)
+
+        handle = lib()
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m vortex_b200.build`")
+        spec = importlib.util.spec_from_file_location("_vtx_host", HOST_PATH)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        if mod.abi_version() != header_abi_version():
+            raise RuntimeError(f"{HOST_PATH} was built for ABI version {mod.abi_version()}: rebuild it with "
+                               "`python -m vortex_b200.build`")
+        mod.bind(*(C.cast(getattr(handle, n), _p).value for n in
+                   ("vtx_decode_layer", "vtx_fused_fir_fwd", "vtx_fused_iir_fwd", "vtx_fused_iir_scratch_bytes", "vtx_last_error")))
+        _host = mod
+    return _host
 
 
 def last_error() -> str:

@@ -1,4 +1,5 @@
-"""Builds ``vortex_b200/lib/libvortex_b200.so`` from ``vortex_b200/csrc/*.cu`` with nvcc for sm_100a.
+"""Builds ``vortex_b200/lib/libvortex_b200.so`` from ``vortex_b200/csrc/*.cu`` with nvcc for sm_100a, and the host
+module ``vortex_b200/lib/_vtx_host.so`` from ``csrc/host.cpp`` with g++ against torch's headers.
 
     python -m vortex_b200.build [--force] [--verbose]
 
@@ -20,6 +21,7 @@ CSRC = os.path.join(PKG, "csrc")
 LIBDIR = os.path.join(PKG, "lib")
 OBJDIR = os.path.join(LIBDIR, "obj")
 LIB = os.path.join(LIBDIR, "libvortex_b200.so")
+HOST_SRC, HOST_LIB = os.path.join(CSRC, "host.cpp"), os.path.join(LIBDIR, "_vtx_host.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -67,11 +69,36 @@ def _compile(src: str, force: bool, verbose: bool) -> tuple[str, bool, str]:
     return obj, True, r.stderr if verbose else ""
 
 
+def _build_host(force: bool) -> None:
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension as ext
+
+    stamp = os.path.join(OBJDIR, "host.sha")
+    want = _digest([HOST_SRC, os.path.join(os.path.dirname(PKG), "include", "vortex_b200.h")]) + torch.__version__ + sysconfig.get_python_version()
+    if not force and os.path.exists(HOST_LIB) and os.path.exists(stamp) and open(stamp).read() == want:
+        return
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    libdir = os.path.join(os.path.dirname(torch.__file__), "lib")
+    inc = [*ext.include_paths(), os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-w", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{d}" for d in inc), HOST_SRC,
+           "-o", HOST_LIB, f"-L{libdir}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for {HOST_SRC}:\n{r.stdout}\n{r.stderr}")
+    with open(stamp, "w") as f:
+        f.write(want)
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OBJDIR, exist_ok=True)
     srcs = sources()
-    with cf.ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
+    with cf.ThreadPoolExecutor(max_workers=min(8, len(srcs)) + 1) as ex:
+        host = ex.submit(_build_host, force)
         results = list(ex.map(lambda s: _compile(s, force, verbose), srcs))
+        host.result()
     objs = [o for o, _, _ in results]
     if verbose:
         for _, _, log in results:

@@ -270,38 +270,8 @@ def fused_fir_fwd(u: torch.Tensor, w3, b3, h, bias, D: int, *, taps: int, bias_m
 
     ``hist_rows`` = H > 0 (chunked prefill): ``u`` is a view whose H preceding rows in memory (same row pitch) hold
     the sequence's earlier projection rows, H >= K + 1; the caches returned are then always full."""
-    _need_cuda(u, w3, b3, h, bias)
-    if u.stride(2) != 1:
-        if hist_rows:
-            raise ValueError("hist_rows needs u with unit channel stride (a view into the buffer that holds the history)")
-        u = u.contiguous()
-    B, L, C3 = u.shape
-    if C3 != 3 * D:
-        raise ValueError(f"expected {3 * D} packed channels, got {C3}")
-    w3 = _param(w3, u).reshape(C3, -1)
-    h = _param(h, u)
-    G = h.shape[0]
-    h = h.reshape(G, -1)
-    K, K3 = h.shape[1], w3.shape[1]
-    b3, bias = _param(b3, u), _param(bias, u)
-    y = torch.empty(B, L, D, device=u.device, dtype=u.dtype)
-    if hist_rows and u.storage_offset() < hist_rows * u.stride(1):
-        raise ValueError(f"hist_rows={hist_rows}: u starts {u.storage_offset() // max(u.stride(1), 1)} rows into its storage")
-    n3, ns = (K3 - 1, K - 1) if hist_rows else (min(L, K3 - 1), min(L, K - 1))
-    fs = torch.empty(B, C3, n3, device=u.device, dtype=u.dtype) if want_state else None
-    ist = torch.empty(B, D, ns, device=u.device, dtype=u.dtype) if want_state else None
-    p = _lib.FusedFirParams(
-        u=_ptr(u), u_stride_b=u.stride(0), u_stride_l=u.stride(1), w3=_ptr(w3), w3_dtype=_code(w3),
-        b3=_ptr(b3), b3_dtype=_code(b3) if b3 is not None else 0, h=_ptr(h), h_dtype=_code(h),
-        bias=_ptr(bias), bias_dtype=_code(bias) if bias is not None else 0,
-        y=_ptr(y), y_stride_b=L * D, y_stride_l=D,
-        fir_state=_ptr(fs) if (fs is not None and fs.numel()) else None,
-        inner_state=_ptr(ist) if (ist is not None and ist.numel()) else None,
-        B=B, L=L, D=D, G=G, K3=K3, K=K, layout=LAYOUTS[layout], num_heads=num_heads, flip_x1x2=int(flip),
-        taps=taps, bias_mode=bias_mode if bias is not None else BIAS_NONE, io_dtype=_code(u), u_hist_rows=hist_rows)
-    with _on(u):
-        _lib.check(_lib.lib().vtx_fused_fir_fwd(C.byref(p), _stream(u)))
-    return y, fs, ist
+    return _lib.host().fused_fir_fwd(u, w3, b3, h, bias, D, taps, bias_mode, LAYOUTS[layout], num_heads, bool(flip),
+                                     bool(want_state), hist_rows)
 
 
 # ----------------------------------------------------------------------------------------------
@@ -335,54 +305,8 @@ def fused_iir_fwd(u: torch.Tensor, w3, log_poles, residues, bias, D: int, *, lay
     ``fir_state_in`` ([B, 3D, 2]) continue an earlier call (chunked prefill).  ``hist_rows`` = H >= 2 instead of
     ``fir_state_in``: ``u`` is a view whose H preceding rows in memory (same row pitch) hold the sequence's earlier
     projection rows; with it, and L a multiple of 384, a continued call stays on the tensor-core kernel."""
-    _need_cuda(u, w3, residues, bias, b3, state_in, fir_state_in)
-    if u.stride(2) != 1:
-        if hist_rows:
-            raise ValueError("hist_rows needs u with unit channel stride (a view into the buffer that holds the history)")
-        u = u.contiguous()
-    if hist_rows:
-        if hist_rows < 2 or fir_state_in is not None:
-            raise ValueError("hist_rows must be >= 2 and excludes fir_state_in")
-        if u.storage_offset() < hist_rows * u.stride(1):
-            raise ValueError(f"hist_rows={hist_rows}: u starts {u.storage_offset() // max(u.stride(1), 1)} rows into its storage")
-    B, L, C3 = u.shape
-    if C3 != 3 * D:
-        raise ValueError(f"expected {3 * D} packed channels, got {C3}")
-    w3 = _param(w3, u).reshape(C3, -1)
-    bias, b3 = _param(bias, u), _param(b3, u)
-    m, keep = _modal(log_poles, residues, u, theta, res_im)
-    cplx = theta is not None
-    if out is None:
-        y = torch.empty(B, L, D, device=u.device, dtype=u.dtype)
-    else:       # a [B, L, D] view with unit channel stride (e.g. a range of rows of a larger output)
-        if tuple(out.shape) != (B, L, D) or out.dtype != u.dtype or out.stride(2) != 1 or out.device != u.device:
-            raise ValueError("out must be a [B, L, D] tensor of u's dtype and device with unit channel stride")
-        y = out
-    st = None
-    if want_state:
-        st = torch.empty((B, D, m.S, 2) if cplx else (B, D, m.S), device=u.device, dtype=torch.float32)
-    if state_in is not None:
-        if tuple(state_in.shape) != ((B, D, m.S, 2) if cplx else (B, D, m.S)):
-            raise ValueError(f"state_in has shape {tuple(state_in.shape)}")
-        state_in = state_in.to(torch.float32).contiguous()
-    if fir_state_in is not None:
-        if tuple(fir_state_in.shape) != (B, C3, 2):
-            raise ValueError(f"fir_state_in has shape {tuple(fir_state_in.shape)}, expected {(B, C3, 2)}")
-        fir_state_in = fir_state_in.contiguous()
-    p = _lib.FusedIirParams(
-        u=_ptr(u), u_stride_b=u.stride(0), u_stride_l=u.stride(1), w3=_ptr(w3), w3_dtype=_code(w3),
-        b3=_ptr(b3), b3_dtype=_code(b3) if b3 is not None else 0,
-        modal=m, bias=_ptr(bias), bias_dtype=_code(bias) if bias is not None else 0,
-        y=_ptr(y), y_stride_b=y.stride(0), y_stride_l=y.stride(1), state=_ptr(st), scratch=None, B=B, L=L, D=D, K3=w3.shape[1],
-        layout=LAYOUTS[layout], num_heads=num_heads, flip_x1x2=int(flip), io_dtype=_code(u),
-        state_in=_ptr(state_in), fir_state_in=_ptr(fir_state_in),
-        fir_state_dtype=_code(fir_state_in) if fir_state_in is not None else 0, u_hist_rows=int(hist_rows))
-    nscratch = _lib.lib().vtx_fused_iir_scratch_bytes(C.byref(p))
-    scratch = torch.empty(nscratch, device=u.device, dtype=torch.uint8) if nscratch > 0 else None
-    p.scratch = _ptr(scratch)
-    with _on(u):
-        _lib.check(_lib.lib().vtx_fused_iir_fwd(C.byref(p), _stream(u)))
-    del keep
+    y, st = _lib.host().fused_iir_fwd(u, w3, log_poles, residues, bias, D, LAYOUTS[layout], num_heads, bool(flip), theta,
+                                      res_im, bool(want_state), b3, state_in, fir_state_in, hist_rows, out)
     return (y, st) if want_state else y
 
 
@@ -632,48 +556,8 @@ def decode_layer(u, w3, b3, fir_state, D, *, h=None, inner_state=None, bias=None
 
     FIR layers pass h / inner_state; the long (modal) layer passes log_poles / residues / iir_state.
     Returns (y, new_fir_state fp32, new_inner_or_iir_state)."""
-    _need_cuda(u, w3, fir_state)
-    u = u.contiguous()
-    B, C3 = u.shape
-    if C3 != 3 * D:
-        raise ValueError(f"expected {3 * D} packed channels, got {C3}")
-    w3 = _param(w3, u).reshape(C3, -1)
-    K3 = w3.shape[1]
-    b3, bias = _param(b3, u), _param(bias, u)
-    fs = fir_state.contiguous()
-    if fs.shape[-1] != K3 - 1:
-        raise NotImplementedError("decode_layer needs a full featurizer cache (prompt of at least K3-1 tokens)")
-    fs_out = torch.empty(B, C3, K3 - 1, device=u.device, dtype=torch.float32)
-    y = torch.empty(B, D, device=u.device, dtype=u.dtype)
-    p = _lib.DecodeLayerParams(
-        u=_ptr(u), w3=_ptr(w3), w3_dtype=_code(w3), b3=_ptr(b3), b3_dtype=_code(b3) if b3 is not None else 0,
-        fir_state_in=_ptr(fs), fir_state_dtype=_code(fs), fir_state_out=_ptr(fs_out), bias=_ptr(bias),
-        bias_dtype=_code(bias) if bias is not None else 0, y=_ptr(y), B=B, D=D, K3=K3, layout=LAYOUTS[layout],
-        num_heads=num_heads, flip_x1x2=int(flip), flip_filter=int(flip_filter), io_dtype=_code(u))
-    keep = None
-    if h is not None:
-        h = _param(h, u)
-        G = h.shape[0]
-        h = h.reshape(G, -1)
-        K = h.shape[1]
-        ins = inner_state.contiguous()
-        if ins.shape[-1] != K - 1:
-            raise NotImplementedError("decode_layer needs a full inner cache (prompt of at least K-1 tokens)")
-        new_state = torch.empty(B, D, K - 1, device=u.device, dtype=torch.float32)
-        p.h, p.h_dtype, p.G, p.K = _ptr(h), _code(h), G, K
-        p.inner_state_in, p.inner_state_dtype, p.inner_state_out = _ptr(ins), _code(ins), _ptr(new_state)
-        p.bias_mode = (BIAS_GATED if gated_bias else BIAS_ADD) if bias is not None else BIAS_NONE
-    else:
-        m, keep = _modal(log_poles, residues, u, theta, res_im)
-        st = iir_state.contiguous()
-        if st.dtype != torch.float32:
-            st = st.float()
-        new_state = torch.empty_like(st)
-        p.modal, p.K, p.G = m, 0, m.G
-        p.iir_state_in, p.iir_state_out = _ptr(st), _ptr(new_state)
-    with _on(u):
-        _lib.check(_lib.lib().vtx_decode_layer(C.byref(p), _stream(u)))
-    return y, fs_out, new_state
+    return _lib.host().decode_layer(u, w3, b3, fir_state, D, h, inner_state, bias, bool(flip_filter), bool(gated_bias),
+                                    log_poles, residues, iir_state, theta, res_im, LAYOUTS[layout], num_heads, bool(flip))
 
 
 def iir_fwd_noalloc(z_pre: torch.Tensor, log_poles, residues, bias, D: int, y: torch.Tensor, state: Optional[torch.Tensor],
