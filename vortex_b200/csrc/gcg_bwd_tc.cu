@@ -18,7 +18,7 @@
 //
 // What bounds it: 10 bytes in and 6 bytes out per element (B=2, L=8192, D=4096: 1.07 GB = 164 us at 6.54 TB/s), i.e. 2900
 // cycles per chunk and SM, of which the tensor pipe needs 16 x 85 (dz) + 8 x 128 (dw) and shared memory about as many.
-// Measured: 307 us with the fp32 accumulator's launch, the fp32 kernels 1290 us; B=4: 529 us = 4.1 TB/s.
+// Measured: 277 us with the launch that clears the fp32 accumulator, the fp32 kernels 1290 us; B=4: 495 us = 4.3 TB/s.
 // Everything arrives by TMA: with 224 KB of the SM carved out as shared memory L1 holds some 220 lines, so plain loads of
 // 32-byte row pieces kept 7 KB in flight (first version: 18000 cycles per chunk, 700 us).
 //
@@ -47,7 +47,9 @@ constexpr int NG = 2, NZ = 3;                      // tile rings: g2 is consumed
 constexpr int NXS = 4, NDS = 3;                    // stages of (x, B), held until the epilogue is done, and of (dy, C, y2)
 constexpr int X_STAGE = 2 * NS * BOX, D_STAGE = 3 * NS * BOX;
 constexpr int OFF_Z = 0, OFF_G = OFF_Z + NZ * TILE, OFF_X = OFF_G + NG * TILE, OFF_D = OFF_X + NXS * X_STAGE;
-constexpr int OFF_TAPS = OFF_D + NDS * D_STAGE, OFF_BARS = OFF_TAPS + 384 * 2;
+constexpr int RUNS = 4, RUN = 40;                  // sums along the anti-diagonals of W: runs per warp, columns per run
+constexpr int RUN_LAGS = RUN + 31;                 // lags a run contributes to
+constexpr int OFF_TAPS = OFF_D + NDS * D_STAGE, OFF_RUNS = OFF_TAPS + 384 * 2, OFF_BARS = OFF_RUNS + 4 * RUNS * RUN_LAGS * 4;
 constexpr int NBARS = 2 * (NG + NZ + NXS + NDS) + 4 + 3;
 constexpr int SMEM_BYTES = OFF_BARS + NBARS * 8 + 16 + 1024;
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
@@ -301,35 +303,47 @@ __global__ void __launch_bounds__(THREADS, 1) gcg_bwd_tc_kernel(const __grid_con
             // Anti-diagonals of W: row i (g2 at time 127 - i of the chunk) and column c (z at time c - 128 of it) meet at lag
             // 255 - i - c, so a sum that moves one lane up per column to the left stays on its lag.  Columns 96 - 32 e ..
             // 255 - 32 e hold every lag 0..127 of this warp's rows; four independent runs of 40 columns hide the shuffle's
-            // latency.  What leaves lane 31 (and what a run still holds at its end) is added to the group's dh.
+            // latency.  Run q's lag 40 q - 31 + m leaves lane 31 at its column m, the last 31 lags sit in the lanes below
+            // at its end: all go to shared memory, and one sum over the runs is added to the group's dh.  (Adding each value
+            // to dh where it left lane 31 took 13 K cycles per item, most of the gap between two items.)
             {
-                float* dh = a.dh + (int64_t)((unsigned)(g * CH) / (unsigned)a.dg) * K;
-                float run[4] = {0.f, 0.f, 0.f, 0.f};
+                float* const sums = reinterpret_cast<float*>(smp(OFF_RUNS)) + e * RUNS * RUN_LAGS;
+                float run[RUNS] = {0.f, 0.f, 0.f, 0.f};
                 const int top = 255 - 32 * e;                      // first column of run 0; run q starts 40 q further left
 #pragma unroll 1
-                for (int c0 = 0; c0 < 40; c0 += 8) {
-                    uint32_t w8[4][8];
+                for (int c0 = 0; c0 < RUN; c0 += 8) {
+                    uint32_t w8[RUNS][8];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) tmem_ld8(lane_base + W_COL + (uint32_t)(top - 40 * q - c0 - 7), w8[q]);
+                    for (int q = 0; q < RUNS; ++q) tmem_ld8(lane_base + W_COL + (uint32_t)(top - RUN * q - c0 - 7), w8[q]);
                     tmem_ld8_wait(w8[0], w8[1]);
                     tmem_ld8_wait(w8[2], w8[3]);
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) {
+                        for (int q = 0; q < RUNS; ++q) {
                             const float up = __shfl_up_sync(0xffffffffu, run[q], 1);
                             run[q] = (lane ? up : 0.f) + __uint_as_float(w8[q][7 - j]);
-                            const int lag = 255 - (e * 32 + 31) - (top - 40 * q - c0 - j);
-                            if (lane == 31 && lag >= 0 && lag < K) atomicAdd(dh + (K - 1 - lag), run[q]);
+                            if (lane == 31) sums[q * RUN_LAGS + c0 + j] = run[q];
                         }
                     }
                 }
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int lag = 255 - i - (top - 40 * q - 39);
-                    if (lane < 31 && lag >= 0 && lag < K) atomicAdd(dh + (K - 1 - lag), run[q]);
-                }
+                for (int q = 0; q < RUNS; ++q)
+                    if (lane < 31) sums[q * RUN_LAGS + RUN_LAGS - 1 - lane] = run[q];
                 tc_fence_before();
+                __syncwarp();
+                float* const dh = a.dh + (int64_t)((unsigned)(g * CH) / (unsigned)a.dg) * K;
+#pragma unroll
+                for (int lag = lane; lag < CHUNK; lag += 32) {
+                    float v = 0.f;
+#pragma unroll
+                    for (int q = 0; q < RUNS; ++q) {
+                        const int m = lag - RUN * q + 31;
+                        if (m >= 0 && m < RUN_LAGS) v += sums[q * RUN_LAGS + m];
+                    }
+                    if (lag < K) atomicAdd(dh + (K - 1 - lag), v);
+                }
+                __syncwarp();
             }
             if (t + 1 < nmine && !expand(t + 1)) ok = false;
         }
