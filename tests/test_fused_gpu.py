@@ -646,6 +646,26 @@ def test_launch_count_follows_the_kernels_a_call_launches():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("io", ["bf16", "f32"])
+@pytest.mark.parametrize("B", [19, 21, 64])
+def test_decode_long_filter_many_sequences(io, B):
+    """The one-token long-filter layer with several batch elements per quad (enough rows for more than one round of
+    blocks, batches that are no multiple of four among them) against the same rows a few sequences at a time: same bits."""
+    from vortex_b200 import ops
+
+    D, S = 4096, 16
+    g = torch.Generator(device="cuda").manual_seed(B)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    u, fs, st = r(B, 3 * D).to(DT[io]), r(B, 3 * D, 2), r(B, D, S)
+    w3, Dp, lp, R = r(3 * D, 1, 3).to(DT[io]), r(D).to(DT[io]), -0.1 * r(D, S, 1).abs(), r(D, S)
+    one = lambda a, b: ops.decode_layer(u[a:b], w3, None, fs[a:b], D, log_poles=lp, residues=R, bias=Dp, iir_state=st[a:b])  # noqa: E731
+    got = one(0, B)
+    parts = [one(a, min(a + 5, B)) for a in range(0, B, 5)]
+    for i, t in enumerate(got):
+        assert torch.equal(t, torch.cat([p[i] for p in parts]))
+
+
+@pytest.mark.gpu
 def test_prefill_caches_of_walks_with_several_items():
     """The inner caches of a call whose CTAs walk several items each, the last chunks of the sequences among the first of
     them: every cached product of every sequence, in calls repeated on the same input (a slot handed to the front end

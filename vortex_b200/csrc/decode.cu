@@ -595,55 +595,78 @@ __global__ void __launch_bounds__(256) decode_iir_tile_kernel(vtx_decode_layer_p
 // Modal layer with real poles when the modal systems are not shared by whole tiles of 8 channels (Evo 2: one system
 // per channel): four lanes per row, each with four of the row's 16 states as one 16-byte load and store; the row's
 // poles and residues are read the same way.  Three of the four lanes do one packed channel of the featurizer each.
-template <typename T>
+// NB: batch elements per quad.  A row is one round trip to memory; once the rows of a launch make more than one round of
+// resident blocks, a quad takes four of them, all loads in flight, on one evaluation of the poles (B=64, D=4096, 48 MB:
+// 10.5 us, 3.5 rounds of single rows: 24 us).
+template <typename T, int NB>
 __global__ void __launch_bounds__(256) decode_iir_quad_kernel(vtx_decode_layer_params p) {
-    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t row = tid >> 2;
-    const int part = (int)(tid & 3);
-    if (row >= p.B * p.D) return;                  // rows are whole quads: a quad leaves together
+    const int64_t quad = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+    const int part = (int)(threadIdx.x & 3);
+    const int64_t b0 = div32(quad, p.D) * NB, d = quad - b0 / NB * p.D;
+    if (b0 >= p.B) return;                         // (a quad leaves together)
     const unsigned mask = 0xfu << ((threadIdx.x & 31) & ~3);
-    const int64_t b = div32(row, p.D), d = row - b * p.D, g = div32(d, div32(p.D, p.modal.G));
-    // state and parameters first: the longest latencies
-    const float4 s = reinterpret_cast<const float4*>(p.iir_state_in + row * 16)[part];
+    const int64_t g = div32(d, div32(p.D, p.modal.G));
+    // every load of the quad's rows and of its parameters before the first use (raw parameter bits: no dtype branch in
+    // between); rows past the last batch element read the first one's and store nothing
+    float4 s[NB];
+    float2 st[NB];
+    T xr[NB];
+    const QkvMap map = qkv_map(p);
+    int64_t ch[3];
+    map.get(d, ch[0], ch[1], ch[2]);
+    const int64_t c = part == 0 ? ch[0] : part == 1 ? ch[1] : ch[2];
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+        const int64_t b = b0 + j < p.B ? b0 + j : b0;
+        s[j] = reinterpret_cast<const float4*>(p.iir_state_in + (b * p.D + d) * 16)[part];
+        if (part < 3) {
+            st[j] = *reinterpret_cast<const float2*>(static_cast<const float*>(p.fir_state_in) + (b * 3 * p.D + c) * 2);
+            xr[j] = static_cast<const T*>(p.u)[b * 3 * p.D + c];
+        }
+    }
     const float4 lp = reinterpret_cast<const float4*>(static_cast<const float*>(p.modal.log_poles) + g * 16)[part];
     const float4 rr = reinterpret_cast<const float4*>(static_cast<const float*>(p.modal.res_re) + g * 16)[part];
-    float z = 0.f;
     const uint32_t draw = (part == 0 && p.bias) ? ld_raw(p.bias, p.bias_dtype == VTX_F32, d) : 0u;
+    const bool wide = p.w3_dtype == VTX_F32;
+    uint32_t wr[3] = {0, 0, 0}, b3r = 0;
     if (part < 3) {
-        const QkvMap map = qkv_map(p);
-        int64_t ch[3];
-        map.get(d, ch[0], ch[1], ch[2]);
-        const int64_t c = part == 0 ? ch[0] : part == 1 ? ch[1] : ch[2], so = (b * 3 * p.D + c) * 2;
-        // every load of the featurizer step before the first use (raw parameter bits: no dtype branch in between)
-        const float2 st = *reinterpret_cast<const float2*>(static_cast<const float*>(p.fir_state_in) + so);
-        const T xr = static_cast<const T*>(p.u)[b * 3 * p.D + c];
-        const bool wide = p.w3_dtype == VTX_F32;
-        const uint32_t w0 = ld_raw(p.w3, wide, c * 3), w1 = ld_raw(p.w3, wide, c * 3 + 1), w2 = ld_raw(p.w3, wide, c * 3 + 2);
-        const uint32_t b3r = p.b3 ? ld_raw(p.b3, p.b3_dtype == VTX_F32, c) : 0u;
-        const float x = to_f32<T>(xr);
-        float acc = cvt_raw(w2, p.w3_dtype) * x;
-        acc = fmaf(st.x, cvt_raw(w0, p.w3_dtype), acc);
-        acc = fmaf(st.y, cvt_raw(w1, p.w3_dtype), acc);
-        *reinterpret_cast<float2*>(p.fir_state_out + so) = make_float2(st.y, x);
-        if (p.b3) acc += cvt_raw(b3r, p.b3_dtype);
-        z = round_io<T>(acc);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) wr[i] = ld_raw(p.w3, wide, c * 3 + i);
+        b3r = p.b3 ? ld_raw(p.b3, p.b3_dtype == VTX_F32, c) : 0u;
     }
-    const float q = __shfl_sync(mask, z, 0, 4), k = __shfl_sync(mask, z, 1, 4), v = __shfl_sync(mask, z, 2, 4);
-    const float kv = round_io<T>(k * v);
-    float4 n;
-    n.x = fmaf(expf(lp.x), s.x, kv);
-    n.y = fmaf(expf(lp.y), s.y, kv);
-    n.z = fmaf(expf(lp.z), s.z, kv);
-    n.w = fmaf(expf(lp.w), s.w, kv);
-    reinterpret_cast<float4*>(p.iir_state_out + row * 16)[part] = n;
-    float sum = fmaf(rr.x, n.x, fmaf(rr.y, n.y, fmaf(rr.z, n.z, rr.w * n.w)));
-    sum += __shfl_xor_sync(mask, sum, 1, 4);
-    sum += __shfl_xor_sync(mask, sum, 2, 4);
-    if (part == 0) {
-        const float bias = p.bias ? cvt_raw(draw, p.bias_dtype) : 0.f;
-        float skip = bias * kv;
-        if (p.bias && p.bias_dtype != VTX_F32) skip = round_io<T>(skip);
-        static_cast<T*>(p.y)[row] = from_f32<T>(q * (sum + skip));
+    const float w0 = cvt_raw(wr[0], p.w3_dtype), w1 = cvt_raw(wr[1], p.w3_dtype), w2 = cvt_raw(wr[2], p.w3_dtype);
+    const float ex = expf(lp.x), ey = expf(lp.y), ez = expf(lp.z), ew = expf(lp.w);
+    const float bias = p.bias ? cvt_raw(draw, p.bias_dtype) : 0.f;
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+        const bool on = b0 + j < p.B;
+        const int64_t b = b0 + j, row = b * p.D + d;
+        float z = 0.f;
+        if (part < 3) {
+            const float x = to_f32<T>(xr[j]);
+            float acc = w2 * x;
+            acc = fmaf(st[j].x, w0, acc);
+            acc = fmaf(st[j].y, w1, acc);
+            if (on) *reinterpret_cast<float2*>(p.fir_state_out + (b * 3 * p.D + c) * 2) = make_float2(st[j].y, x);
+            if (p.b3) acc += cvt_raw(b3r, p.b3_dtype);
+            z = round_io<T>(acc);
+        }
+        const float q = __shfl_sync(mask, z, 0, 4), k = __shfl_sync(mask, z, 1, 4), v = __shfl_sync(mask, z, 2, 4);
+        const float kv = round_io<T>(k * v);
+        float4 n;
+        n.x = fmaf(ex, s[j].x, kv);
+        n.y = fmaf(ey, s[j].y, kv);
+        n.z = fmaf(ez, s[j].z, kv);
+        n.w = fmaf(ew, s[j].w, kv);
+        if (on) reinterpret_cast<float4*>(p.iir_state_out + row * 16)[part] = n;
+        float sum = fmaf(rr.x, n.x, fmaf(rr.y, n.y, fmaf(rr.z, n.z, rr.w * n.w)));
+        sum += __shfl_xor_sync(mask, sum, 1, 4);
+        sum += __shfl_xor_sync(mask, sum, 2, 4);
+        if (part == 0 && on) {
+            float skip = bias * kv;
+            if (p.bias && p.bias_dtype != VTX_F32) skip = round_io<T>(skip);
+            static_cast<T*>(p.y)[row] = from_f32<T>(q * (sum + skip));
+        }
     }
 }
 
@@ -750,7 +773,10 @@ extern "C" int vtx_decode_layer(const vtx_decode_layer_params* p, void* stream) 
                 if (cplx) decode_iir_tile_kernel<T, 8, true><<<(unsigned)nblk, 256, 0, s>>>(*p, (int)tpg, gpb);
                 else decode_iir_tile_kernel<T, 8, false><<<(unsigned)nblk, 256, 0, s>>>(*p, (int)tpg, gpb);
             } else if (quad) {
-                decode_iir_quad_kernel<T><<<(unsigned)ceil_div<int64_t>(rows * 4, 256), 256, 0, s>>>(*p);
+                const int64_t blocks = ceil_div<int64_t>(rows * 4, 256);       // (eight of them fit an SM)
+                if (blocks > kNumSMs * 8)
+                    decode_iir_quad_kernel<T, 4><<<(unsigned)ceil_div<int64_t>(ceil_div<int64_t>(p->B, 4) * p->D * 4, 256), 256, 0, s>>>(*p);
+                else decode_iir_quad_kernel<T, 1><<<(unsigned)blocks, 256, 0, s>>>(*p);
             } else {
                 decode_layer_kernel<T, 16, 1><<<(unsigned)ceil_div<int64_t>(rows * 16, 256), 256, 0, s>>>(*p);
             }
