@@ -67,14 +67,16 @@ constexpr int OFF_RES = OFF_H + CHUNK * 4;                   // float2 [16]: res
 static_assert(OFF_RES + NPOLE * 8 <= OFF_SLOTS + NSLOT * SLOT_BYTES, "set-up tables must fit into a slot");
 constexpr int OFF_DIAG = OFF_SLOTS + NSLOT * SLOT_BYTES;     // float [16]: skip parameters
 constexpr int OFF_BARS = OFF_DIAG + 64;
-constexpr int NBARS = IN_STAGES * 2 + NSLOT * 3 + 2 * 3 + 1;
+constexpr int ND = 3;                      // accumulators: one takes T and Bm, one waits for its states and C S, one is read out
+constexpr int NBARS = IN_STAGES * 2 + NSLOT * 3 + ND * 3 + 1;
 constexpr int SMEM_BYTES = OFF_BARS + NBARS * 8 + 16 + 1024;
 static_assert(OFF_SLOTS % 1024 == 0 && SLOT_BYTES % 1024 == 0 && QH_OFF % 1024 == 0 &&
               SH_OFF % 1024 == 0 && SL_OFF % 1024 == 0, "tiles must be 1024-byte aligned");
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
 // TMEM columns: stacked [T; Bm] head and remainder (96 K elements = 48 columns each), [C; 0] head and remainder
-// (32 K elements = 16 columns each), two accumulators of 128 columns
+// (32 K elements = 16 columns each), three accumulators of 128 columns
 constexpr int A_HI = 0, A_LO = 48, C_HI = 96, C_LO = 112, D_COL = 128, TMEM_COLS = 512;
+static_assert(D_COL + ND * 128 <= TMEM_COLS, "tensor memory");
 constexpr int W_EP = NFE, W_ST = NFE + 3, W_MMA = NFE + 4, W_TMA = NFE + 5, NTMA = 2, W_ST2 = NFE + 7;   // state warps: warp % 4 == 3
 constexpr int THREADS = 32 * 16;
 
@@ -93,6 +95,12 @@ struct Args {
     int64_t hd;
 };
 
+__device__ __forceinline__ uint4 lds16(uint32_t addr) {      // (volatile: issued where it stands)
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+    return v;
+}
+
 template <bool INTERLEAVED, bool SWAP>
 __global__ void __launch_bounds__(THREADS, 1) fused_li_kernel(const __grid_constant__ CUtensorMap tmap, Args a) {
     extern __shared__ uint8_t smem_raw[];
@@ -108,9 +116,9 @@ __global__ void __launch_bounds__(THREADS, 1) fused_li_kernel(const __grid_const
     auto s_full = [&](int sl) { return smem_u32(&bars[BB + 2 * NSLOT + sl]); };           // state warps: chunk-start states in shared memory
     const int BD = BB + 3 * NSLOT;
     auto inc_full = [&](int d) { return smem_u32(&bars[BD + d]); };                       // MMA commit: T/Bm part accumulated
-    auto d_full = [&](int d) { return smem_u32(&bars[BD + 2 + d]); };                     // MMA commit: C S part accumulated too
-    auto d_empty = [&](int d) { return smem_u32(&bars[BD + 4 + d]); };                    // 3 epilogue warps + 2 state warps: accumulator read
-    const uint32_t a_ready = smem_u32(&bars[BD + 6]);                                     // operands expanded, set-up tables no longer needed
+    auto d_full = [&](int d) { return smem_u32(&bars[BD + ND + d]); };                    // MMA commit: C S part accumulated too
+    auto d_empty = [&](int d) { return smem_u32(&bars[BD + 2 * ND + d]); };               // 3 epilogue warps + 2 state warps: accumulator read
+    const uint32_t a_ready = smem_u32(&bars[BD + 3 * ND]);                                // operands expanded, set-up tables no longer needed
 
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     // blockIdx = (time slice, batch element, group), slices of a walk in increasing block order: a slice starts from the
@@ -127,7 +135,7 @@ __global__ void __launch_bounds__(THREADS, 1) fused_li_kernel(const __grid_const
     if (tid == 0) {
         for (int st = 0; st < IN_STAGES; ++st) { mbar_init(in_full(st), NTMA); mbar_init(in_empty(st), NFE / 2); }
         for (int sl = 0; sl < NSLOT; ++sl) { mbar_init(kv_full(sl), NFE); mbar_init(slot_free(sl), 4); mbar_init(s_full(sl), 2); }
-        for (int d = 0; d < 2; ++d) { mbar_init(inc_full(d), 1); mbar_init(d_full(d), 1); mbar_init(d_empty(d), 5); }
+        for (int d = 0; d < ND; ++d) { mbar_init(inc_full(d), 1); mbar_init(d_full(d), 1); mbar_init(d_empty(d), 5); }
         mbar_init(a_ready, NFE + 5);
         fence_mbar_init();
     }
@@ -351,8 +359,8 @@ __global__ void __launch_bounds__(THREADS, 1) fused_li_kernel(const __grid_const
         }
         const int64_t step_pitch = (int64_t)SUPER * a.y_stride_l;
         for (int k = 0; k < nsc; ++k) {
-            const int slot = k % NSLOT, dbuf = k % 2;
-            if (!mbar_wait(d_full(dbuf), (uint32_t)((k / 2) & 1), 5)) break;
+            const int slot = k % NSLOT, dbuf = k % ND;
+            if (!mbar_wait(d_full(dbuf), (uint32_t)((k / ND) & 1), 5)) break;
             tc_fence_after();
             __syncwarp();
             const uint32_t taddr = tmem + ((uint32_t)(e * 32) << 16) + D_COL + dbuf * 128;
@@ -456,8 +464,8 @@ __global__ void __launch_bounds__(THREADS, 1) fused_li_kernel(const __grid_const
             }
         }
         for (int k = 0; k < nsc; ++k) {
-            const int slot = k % NSLOT, dbuf = k % 2;
-            if (!mbar_wait(inc_full(dbuf), (uint32_t)((k / 2) & 1), 12)) break;
+            const int slot = k % NSLOT, dbuf = k % ND;
+            if (!mbar_wait(inc_full(dbuf), (uint32_t)((k / ND) & 1), 12)) break;
             tc_fence_after();
             __syncwarp();
             const uint32_t taddr = tmem + ((uint32_t)CHUNK << 16) + D_COL + dbuf * 128 + 8 * half;
@@ -525,31 +533,47 @@ __global__ void __launch_bounds__(THREADS, 1) fused_li_kernel(const __grid_const
             const uint64_t kv_desc0 = smem_desc(sm_u + OFF_SLOTS + HI_OFF, KV_TILE, 1024, 2);
             const uint64_t s_desc0 = smem_desc(sm_u + OFF_SLOTS + SH_OFF, S_TILE, 1024, 2);
             bool ok = mbar_wait(a_ready, 0, 10);
-            for (int k = 0; k < nsc && ok; ++k) {
-                const int slot = k % NSLOT, dbuf = k % 2;
-                if (!mbar_wait(kv_full(slot), (uint32_t)((k / NSLOT) & 1), 6)) break;
-                if (k >= 2 && !mbar_wait(d_empty(dbuf), (uint32_t)(((k - 2) / 2) & 1), 8)) break;
-                tc_fence_after();
-                const uint32_t d = tmem + D_COL + dbuf * 128;
-                // descriptors of the slot's tiles: the start-address field counts 16-byte units
-                const uint64_t dk = kv_desc0 + (uint64_t)(slot * (SLOT_BYTES / 16)), ds = s_desc0 + (uint64_t)(slot * (SLOT_BYTES / 16));
-                // outputs of the four chunks (lanes 0..95) and their state increments (lanes 96..127)
+            // Two streams of work, whichever is ready: T and Bm of step kt (needs its k*v tile and a free accumulator), C S of
+            // step kc (needs its chunk-start states, which the state warps make from kc's increments).  In a fixed order
+            // one of them waits for the other's operands: T after C S leaves the tensor pipe idle during the state
+            // recurrence, C S after the next T keeps a finished step's slot and accumulator for another period.  (B=1,
+            // L=131072, D=4096: 1194 us; C S between two T 1220, T before C S 1252.)
+            int kt = 0, kc = 0;
+            for (int idle = 0; ok && kc < nsc;) {
+                if (kc < kt && mbar_test_wait(s_full(kc % NSLOT), (uint32_t)((kc / NSLOT) & 1))) {
+                    tc_fence_after();
+                    const int slot = kc % NSLOT, dbuf = kc % ND;
+                    const uint64_t ds = s_desc0 + (uint64_t)(slot * (SLOT_BYTES / 16));
+                    // + C S: contribution of everything before each chunk
 #pragma unroll
-                for (int part = 0; part < 2; ++part)
+                    for (int part = 0; part < 2; ++part)
 #pragma unroll
-                    for (int jj = 0; jj < CHUNK / 16; ++jj)
-                        mma_ts(d, tmem + (part ? A_LO : A_HI) + 8 * jj, dk + (uint64_t)(jj * 128), idesc, (part || jj) ? 1u : 0u);
-                mma_commit(inc_full(dbuf));
-                // + C S: contribution of everything before each chunk
-                if (!mbar_wait(s_full(slot), (uint32_t)((k / NSLOT) & 1), 13)) break;
-                tc_fence_after();
+                        for (int jj = 0; jj < 2; ++jj)
+                            mma_ts(tmem + D_COL + dbuf * 128, tmem + (part ? C_LO : C_HI) + 8 * jj, ds + (uint64_t)(jj * 128), idesc, 1u);
+                    mma_commit(d_full(dbuf));
+                    mma_commit(slot_free(slot));
+                    ++kc;
+                    idle = 0;
+                } else if (kt < nsc && mbar_test_wait(kv_full(kt % NSLOT), (uint32_t)((kt / NSLOT) & 1)) &&
+                           (kt < ND || mbar_test_wait(d_empty(kt % ND), (uint32_t)(((kt - ND) / ND) & 1)))) {
+                    tc_fence_after();
+                    const int slot = kt % NSLOT, dbuf = kt % ND;
+                    // descriptors of the slot's tiles: the start-address field counts 16-byte units
+                    const uint64_t dk = kv_desc0 + (uint64_t)(slot * (SLOT_BYTES / 16));
+                    // outputs of the four chunks (lanes 0..95) and their state increments (lanes 96..127)
 #pragma unroll
-                for (int part = 0; part < 2; ++part)
+                    for (int part = 0; part < 2; ++part)
 #pragma unroll
-                    for (int jj = 0; jj < 2; ++jj)
-                        mma_ts(d, tmem + (part ? C_LO : C_HI) + 8 * jj, ds + (uint64_t)(jj * 128), idesc, 1u);
-                mma_commit(d_full(dbuf));
-                mma_commit(slot_free(slot));
+                        for (int jj = 0; jj < CHUNK / 16; ++jj)
+                            mma_ts(tmem + D_COL + dbuf * 128, tmem + (part ? A_LO : A_HI) + 8 * jj, dk + (uint64_t)(jj * 128), idesc,
+                                   (part || jj) ? 1u : 0u);
+                    mma_commit(inc_full(dbuf));
+                    ++kt;
+                    idle = 0;
+                } else if (++idle == 1 << 26) {
+                    atomicCAS(&g_device_status, 0, 13);
+                    ok = false;
+                }
             }
         }
     } else if (warp < W_TMA + NTMA) {
