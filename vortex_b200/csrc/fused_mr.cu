@@ -47,12 +47,6 @@ constexpr int CHUNK = 128;                 // output samples per MMA chunk
 constexpr int NFE = VTX_MR_NFE;            // front-end warps (two per scheduler: the featurizer chain is latency-bound)
 constexpr int WROWS = CHUNK / NFE;         // rows of a chunk owned by one front-end warp
 constexpr int RB = 8;                      // rows a front-end lane fetches into registers at a time
-constexpr int HROWS = 64;                  // rows per staged box: half a chunk, shared by two front-end warps
-                                           // (the TMA unit retires ~12 boxes per microsecond and SM whatever their
-                                           // size, so boxes are made as tall as the shared-memory budget allows)
-constexpr int BOX_ROWS = HROWS + 2 + (NS - 1);         // featurizer halo + stream skew
-constexpr int BOX_BYTES = BOX_ROWS * 3 * CH * 2;       // 6624
-constexpr int IN_PLANE = (BOX_ROWS * 32 + 127) / 128 * 128;   // q | k | v planes of the non-interleaved layouts (TMA wants 128-byte aligned tiles)
 constexpr float KV_SCALE = 0.015625f, KV_UNSCALE = 64.f;      // k*v crosses shared memory as fp16 scaled by 2^-6
 
 // k*v and q tiles of a chunk: [128 rows (time)][128 B = 64 channels] fp16 with the 128-byte swizzle (16-byte chunk c of
@@ -69,11 +63,19 @@ constexpr int W3S_BYTES = 3 * 3 * CH * 4;  // featurizer taps of a group as fp32
 // Shared-memory plan.  HBM latency under load is ~2 us, so full bandwidth needs ~100 KB in flight per SM: the ring of
 // half-chunk stages (a stage is handed back as soon as its rows sit in registers) gets all the memory the two chunk
 // slots leave.  The planar q | k | v layouts stage three 128-byte aligned planes per box, the interleaved layout one.
-template <bool INTERLEAVED>
+// Rows per staged box: half a chunk, shared by half of the front-end warps.  The TMA unit retires ~12 boxes per microsecond
+// and SM whatever their size; the operator-only variant, with a box per operand and stream, would need all of them at
+// half a chunk (24 per 1.97 us), so it stages whole chunks: 143 instead of 148 us for the training forward (B=2, L=8192,
+// D=4096), 117 instead of 123 us without the saved filter output.
+template <bool INTERLEAVED, bool FEAT>
 struct Lay {
+    static constexpr int HPC = FEAT ? 2 : 1, HROWS = CHUNK / HPC;        // boxes per chunk, rows per box
+    static constexpr int BOX_ROWS = HROWS + 2 + (NS - 1);                // featurizer halo + stream skew
+    static constexpr int BOX_BYTES = BOX_ROWS * 3 * CH * 2;
+    static constexpr int IN_PLANE = (BOX_ROWS * 32 + 127) / 128 * 128;   // q | k | v planes of the non-interleaved layouts (TMA wants 128-byte aligned tiles)
     static constexpr int BOX_STRIDE = INTERLEAVED ? (BOX_BYTES + 127) / 128 * 128 : 3 * IN_PLANE;   // 6656 : 6912
-    static constexpr int IN_STAGES = INTERLEAVED ? 6 : 5;
-    static constexpr int STAGE_BYTES = NS * BOX_STRIDE;           // the four streams' boxes of one half chunk
+    static constexpr int IN_STAGES = INTERLEAVED ? 6 : FEAT ? 5 : 3;
+    static constexpr int STAGE_BYTES = NS * BOX_STRIDE;           // the four streams' boxes of one stage
     static constexpr int OFF_SLOTS = IN_STAGES * STAGE_BYTES;
     static constexpr int OFF_DIAG = OFF_SLOTS + 2 * SLOT_BYTES;
     static constexpr int OFF_TAPS = OFF_DIAG + DIAG_BYTES;
@@ -146,7 +148,8 @@ template <bool INTERLEAVED, bool SWAP, bool FEAT>
 __global__ void __launch_bounds__(THREADS, 1) fused_mr_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmap_k,
                                                               const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ Args a) {
     static_assert(FEAT || (!INTERLEAVED && !SWAP), "the operator-only variant stages three planes");
-    using LY = Lay<INTERLEAVED>;
+    using LY = Lay<INTERLEAVED, FEAT>;
+    constexpr int HPC = LY::HPC, HROWS = LY::HROWS, BOX_BYTES = LY::BOX_BYTES, IN_PLANE = LY::IN_PLANE;
     constexpr int IN_STAGES = LY::IN_STAGES, BOX_STRIDE = LY::BOX_STRIDE, STAGE_BYTES = LY::STAGE_BYTES;
     constexpr int OFF_SLOTS = LY::OFF_SLOTS, OFF_DIAG = LY::OFF_DIAG, OFF_TAPS = LY::OFF_TAPS, OFF_W3S = LY::OFF_W3S;
     extern __shared__ uint8_t smem_raw[];
@@ -184,7 +187,7 @@ __global__ void __launch_bounds__(THREADS, 1) fused_mr_kernel(const __grid_const
 
     // ---------------- setup -------------------------------------------------------------------
     if (tid == 0) {
-        for (int st = 0; st < IN_STAGES; ++st) { mbar_init(in_full(st), NTMA); mbar_init(in_empty(st), NFE / 2); }
+        for (int st = 0; st < IN_STAGES; ++st) { mbar_init(in_full(st), NTMA); mbar_init(in_empty(st), NFE / HPC); }
         for (int sl = 0; sl < 2; ++sl) {
             mbar_init(kv_full(sl), NFE); mbar_init(slot_free(sl), 6); mbar_init(d_full(sl), 1); mbar_init(d_empty(sl), 4);
             mbar_init(a_ready(sl), 4); mbar_init(taps_ready(sl), 4);
@@ -225,14 +228,14 @@ __global__ void __launch_bounds__(THREADS, 1) fused_mr_kernel(const __grid_const
         };
         // lane constants folded into two offsets: the lane's first staged word of a half chunk, and its fp16 pair in row
         // 16 w of a k*v tile (16-byte chunk 2 s + p / 4, bytes 4 (p % 4))
-        const uint32_t lane_box = (uint32_t)(s * BOX_STRIDE + ((w % (NFE / 2)) * WROWS + s) * (INTERLEAVED ? 96 : 32) + (INTERLEAVED ? 12 : 4) * p);
+        const uint32_t lane_box = (uint32_t)(s * BOX_STRIDE + ((w % (NFE / HPC)) * WROWS + s) * (INTERLEAVED ? 96 : 32) + (INTERLEAVED ? 12 : 4) * p);
         const uint32_t lane_kv = (uint32_t)(((s * 2 + p / 4) << 4) + (p % 4) * 4 + w * WROWS * 128);
-        const uint32_t half = (uint32_t)(w / (NFE / 2));
+        const uint32_t half = (uint32_t)(w / (NFE / HPC));
         constexpr int ROWB = INTERLEAVED ? 96 : 32;             // bytes per staged row (per plane in the planar layouts)
         // shared-memory address of this lane's first word of batch hb of chunk k (the box row of the batch's first
         // sample minus the two featurizer history rows; stream s was staged s rows early)
         auto box_addr = [&](uint32_t k, int hb) {
-            const uint32_t stg = (2 * k + half) % IN_STAGES;
+            const uint32_t stg = (HPC * k + half) % IN_STAGES;
             return sm_u + stg * STAGE_BYTES + lane_box + (uint32_t)(hb * RB * ROWB);
         };
         // Volatile loads: they are issued where they stand, one batch ahead of the arithmetic that consumes them, so
@@ -295,8 +298,8 @@ __global__ void __launch_bounds__(THREADS, 1) fused_mr_kernel(const __grid_const
                 asm volatile("st.shared.b32 [%0], %1;" ::"r"(kaddr + (Q_OFF + i * 128)), "r"(qw));
             }
         };
-        auto stage_of = [&](uint32_t k) { return (int)((2 * k + half) % IN_STAGES); };
-        auto stage_parity = [&](uint32_t k) { return ((2 * k + half) / IN_STAGES) & 1u; };
+        auto stage_of = [&](uint32_t k) { return (int)((HPC * k + half) % IN_STAGES); };
+        auto stage_parity = [&](uint32_t k) { return ((HPC * k + half) / IN_STAGES) & 1u; };
 
         // Software pipeline over register batches A (rows 0..RB-1 of the warp's rows) and B (the rest):
         //   fetch B(k) | wait slot | compute A(k) | release stage | wait stage(k+1), fetch A(k+1) | compute B(k) | publish
@@ -579,7 +582,7 @@ __global__ void __launch_bounds__(THREADS, 1) fused_mr_kernel(const __grid_const
             // ======== TMA issue ======================================================================
             tma_prefetch_desc(&tmap);
             if (!FEAT) { tma_prefetch_desc(&tmap_k); tma_prefetch_desc(&tmap_v); }
-            uint32_t nh = 2 * cc;                    // staged half chunks so far
+            uint32_t nh = HPC * cc;                  // stages filled so far
             bool ok = true;
             for (int t = 0; t < nmine && ok; ++t) {
                 // first packed column of the item's group in q | k | v (one contiguous run when interleaved)
@@ -606,8 +609,8 @@ __global__ void __launch_bounds__(THREADS, 1) fused_mr_kernel(const __grid_const
                     row_base[s] = (int)st.ts - CHUNK - 2 - s + a.hist;
                     bidx[s] = (int)st.b;
                 }
-                for (int hh = 0; hh < 2 * nchunk; ++hh, ++nh) {
-                    const int stg = (int)(nh % IN_STAGES), k = hh / 2, h = hh % 2;
+                for (int hh = 0; hh < HPC * nchunk; ++hh, ++nh) {
+                    const int stg = (int)(nh % IN_STAGES), k = hh / HPC, h = hh % HPC;
                     if (nh >= IN_STAGES && !mbar_wait(in_empty(stg), ((nh - IN_STAGES) / IN_STAGES) & 1u, 9)) { ok = false; break; }
                     const uint32_t bar = in_full(stg);
                     mbar_expect_tx(bar, NS / NTMA * BOX_BYTES);
@@ -847,11 +850,11 @@ int fused_mr_tc_fwd(const vtx_fused_fir_params* p, cudaStream_t stream) {
     // the tensor map starts at the first history row (chunked prefill), else at u
     const __nv_bfloat16* u_first = static_cast<const __nv_bfloat16*>(p->u) - p->u_hist_rows * p->u_stride_l;
     if (int rc = make_tmap_3d(&tmap, u_first, VTX_BF16, 3 * p->D, p->L + p->u_hist_rows, p->B, p->u_stride_l, p->u_stride_b,
-                              inter ? 3 * CH : CH, BOX_ROWS, 0, "fused_fir(mr)"))
+                              inter ? 3 * CH : CH, Lay<true, true>::BOX_ROWS, 0, "fused_fir(mr)"))
         return rc;
-    if (!inter) return launch(fused_mr_kernel<false, false, true>, 0, Lay<false>::SMEM_BYTES, tmap, tmap, tmap, a, stream);
-    if (!a.flip) return launch(fused_mr_kernel<true, false, true>, 1, Lay<true>::SMEM_BYTES, tmap, tmap, tmap, a, stream);
-    return launch(fused_mr_kernel<true, true, true>, 2, Lay<true>::SMEM_BYTES, tmap, tmap, tmap, a, stream);
+    if (!inter) return launch(fused_mr_kernel<false, false, true>, 0, Lay<false, true>::SMEM_BYTES, tmap, tmap, tmap, a, stream);
+    if (!a.flip) return launch(fused_mr_kernel<true, false, true>, 1, Lay<true, true>::SMEM_BYTES, tmap, tmap, tmap, a, stream);
+    return launch(fused_mr_kernel<true, true, true>, 2, Lay<true, true>::SMEM_BYTES, tmap, tmap, tmap, a, stream);
 }
 
 }  // namespace vtx
@@ -904,8 +907,8 @@ extern "C" int vtx_gcg_cl_fwd_saving(const vtx_gcg_cl_params* p, void* y2, void*
     const void* ptrs[3] = {p->q, p->k, p->v};
     const int64_t sl[3] = {p->q_stride_l, p->k_stride_l, p->v_stride_l}, sb[3] = {p->q_stride_b, p->k_stride_b, p->v_stride_b};
     for (int i = 0; i < 3; ++i)
-        if (int rc = make_tmap_3d(&tm[i], ptrs[i], VTX_BF16, p->D, p->L, p->B, sl[i], sb[i], CH, BOX_ROWS, 0, "gcg_cl")) return rc;
-    if (int rc = launch(fused_mr_kernel<false, false, false>, 3, Lay<false>::SMEM_BYTES, tm[0], tm[1], tm[2], a, (cudaStream_t)stream))
+        if (int rc = make_tmap_3d(&tm[i], ptrs[i], VTX_BF16, p->D, p->L, p->B, sl[i], sb[i], CH, Lay<false, false>::BOX_ROWS, 0, "gcg_cl")) return rc;
+    if (int rc = launch(fused_mr_kernel<false, false, false>, 3, Lay<false, false>::SMEM_BYTES, tm[0], tm[1], tm[2], a, (cudaStream_t)stream))
         return rc;
     const int64_t ns = p->L < p->K - 1 ? p->L : p->K - 1;
     if (p->state && ns > 0) {
