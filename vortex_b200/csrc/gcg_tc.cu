@@ -16,9 +16,12 @@
 //
 // One persistent CTA per SM, 16 warps: 0-3 front end (k*v of the staged k and v tiles into the chunk's slot, and the
 // inner FIR cache from the last K-1 products of a sequence), 4-11 epilogue (thread = output sample, two warps per TMEM
-// lane quarter with two streams each: TMEM -> skip -> round -> gate, the result written over the q tile in place and
-// stored by TMA in whole 128-byte rows along time; the first four also expand the next item's Toeplitz operand),
-// 12 MMA issue, 13 TMA issue for k and v, 14 TMA issue for q.  q
+// lane quarter with two streams each: TMEM -> skip -> round -> gate, the result written over the q tile in place; the
+// first four also expand the next item's Toeplitz operand), 12 MMA issue, 13 TMA issue for k and v, 14 TMA issue for q,
+// 15 TMA stores of the finished tiles in whole 128-byte rows along time.  The epilogue is what bounds the kernel
+// (configuration B=4, L=8192, D=4096, 128 taps: 276 us with a round trip per channel pair, 251 with a stream's loads
+// together, 213 us = 0.77 of the HBM peak with the stores in a warp of their own; a third k*v slot: 222).  With fewer than
+// three batch elements the 32 boxes of a chunk are as many as the TMA unit retires (B=1, L=4001: 64 -> 51 us).  q
 // never passes through the front end: its tiles stay in their ring until their chunk's outputs have left through
 // them.  All waits are bounded.
 #include <cstdint>
@@ -48,14 +51,14 @@ constexpr int TAPS_BYTES = 2 * 384 * 2;       // zero-padded taps, bf16; two buf
 constexpr int OFF_DIAG = OFF_TAPS + TAPS_BYTES;
 constexpr int DIAG_BYTES = 2 * 64;            // skip parameters of the block's 16 channels, fp32; two buffers
 constexpr int OFF_BARS = OFF_DIAG + DIAG_BYTES;
-constexpr int NBARS = 2 * NKV + 2 * NQ + 2 * NSLOT + 2 * 5;
+constexpr int NBARS = 2 * NKV + 3 * NQ + 2 * NSLOT + 2 * 4;
 constexpr int OFF_TSLOT = OFF_BARS + NBARS * 8;
 constexpr int SMEM_BYTES = OFF_TSLOT + 16 + 1024;
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
 static_assert(OFF_Q % 1024 == 0 && OFF_SLOTS % 1024 == 0, "tiles are 1024-byte aligned (swizzle atoms)");
 constexpr int TMEM_COLS = 512;                // Toeplitz operand of item t at 128 (t & 1); accumulator buffer b at 256 + 64 b
 constexpr int D_COL = 256;
-constexpr int NFE = 4, W_EP = 4, NEP = 8, W_MMA = 12, W_TKV = 13, W_TQ = 14;   // NEP epilogue warps: two per TMEM lane quarter
+constexpr int NFE = 4, W_EP = 4, NEP = 8, W_MMA = 12, W_TKV = 13, W_TQ = 14, W_ST = 15;   // NEP epilogue warps: two per TMEM lane quarter
 constexpr int THREADS = 16 * 32;
 
 struct Args {
@@ -124,7 +127,7 @@ gcg_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ C
     auto d_empty = [&](int i) { return bar_u + 8u * (uint32_t)(BC + 2 + i); };
     auto a_ready = [&](int i) { return bar_u + 8u * (uint32_t)(BC + 4 + i); };
     auto taps_ready = [&](int i) { return bar_u + 8u * (uint32_t)(BC + 6 + i); };
-    auto y_ready = [&](int i) { return bar_u + 8u * (uint32_t)(BC + 8 + i); };        // a chunk's outputs written (4 epilogue warps)
+    auto y_ready = [&](int i) { return bar_u + 8u * (uint32_t)(BC + 8 + i); };        // the outputs in this q stage are written (8 epilogue warps)
 
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     const int ncta = (int)gridDim.x;
@@ -136,10 +139,10 @@ gcg_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ C
 
     if (tid == 0) {
         for (int i = 0; i < NKV; ++i) { mbar_init(kvin_full(i), 1); mbar_init(kvin_empty(i), NFE); }
-        for (int i = 0; i < NQ; ++i) { mbar_init(q_full(i), 1); mbar_init(q_empty(i), 1); }
+        for (int i = 0; i < NQ; ++i) { mbar_init(q_full(i), 1); mbar_init(q_empty(i), 1); mbar_init(y_ready(i), NEP); }
         for (int i = 0; i < NSLOT; ++i) { mbar_init(kv_full(i), NFE); mbar_init(kv_free(i), NEP + 1); }
         for (int i = 0; i < 2; ++i) {
-            mbar_init(d_full(i), 1); mbar_init(d_empty(i), NEP); mbar_init(a_ready(i), 4); mbar_init(taps_ready(i), 4); mbar_init(y_ready(i), NEP);
+            mbar_init(d_full(i), 1); mbar_init(d_empty(i), NEP); mbar_init(a_ready(i), 4); mbar_init(taps_ready(i), 4);
         }
         fence_mbar_init();
     }
@@ -251,21 +254,10 @@ gcg_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ C
             return true;
         };
         bool ok = sh == 0 ? expand(0) : true;      // (the first four warps expand the operands)
-        int pending = -1;          // q stage whose tile of outputs the TMA unit may still be reading
         for (int t = 0; t < nmine && ok; ++t) {
             const int blk = item_blk(t);
             const float* dsk = reinterpret_cast<const float*>(smp(OFF_DIAG + (t & 1) * 64));
-            // The outputs of a chunk replace the q tile in place (same column, same sample), and one thread hands the
-            // tile to the TMA unit: boxes of [16 channels x 64 samples] (x 4 batch elements) stored with whole 128-byte
-            // rows along time; samples past the end of the sequence are clipped by the tensor map.
-            int x0[NS], bi[NS];
-            bool act[NS];
-#pragma unroll
-            for (int s = 0; s < NS; ++s) {
-                const Stream st = stream_of(a, item_quad(t), s);
-                x0[s] = (int)st.ts; bi[s] = (int)st.b; act[s] = st.active;
-            }
-            const int64_t d0 = (int64_t)blk * CH;
+            // The outputs of a chunk replace the q tile in place (same column, same sample); the store warp takes it from there.
             // The item's halo chunk has no epilogue, but its arrival must not count for the chunk before it in the slot, which
             // another epilogue warp may still be reading: once the halo's tile is full, that chunk has been freed by all.
             if (!mbar_wait(kv_full(cc % NSLOT), (cc / NSLOT) & 1u, 44)) { ok = false; break; }
@@ -289,11 +281,24 @@ gcg_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ C
                     asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
                     return (uint32_t)v;
                 };
-                // (rolled over the streams: the unrolled form did not fit the instruction cache next to the other roles)
+                // (rolled over the streams: the unrolled form did not fit the instruction cache next to the other roles).  A
+                // stream's 32 samples of q and k*v are requested together, before its accumulators are waited for, and its
+                // outputs stored together: two warps per scheduler do this work, and pair by pair -- load, gate, store --
+                // every pair paid the round trip of its loads (3600 of 4250 cycles per chunk, which everything else then
+                // waited for).
+                const bool skip = a.bias_mode == VTX_BIAS_GATED;
 #pragma unroll 1
                 for (int s = 2 * sh; s < 2 * sh + 2; ++s) {
-                    uint32_t acc[16];
+                    uint32_t acc[16], qv[16], kvv[16];
                     tmem_ld16(taddr + s * 16, acc);
+                    const uint32_t qs_u = q_u + (uint32_t)(s * CH * 128), kvs_u = kv_u + (uint32_t)(s * CH * 128);
+                    // (16 s + c) & 7 == c & 7: the swizzle term of a column does not depend on the stream
+#pragma unroll
+                    for (int c = 0; c < CH; ++c) qv[c] = lds16(qs_u + xo[c & 7] + (uint32_t)(c * 128));
+                    if (skip) {
+#pragma unroll
+                        for (int c = 0; c < CH; ++c) kvv[c] = lds16(kvs_u + xo[c & 7] + (uint32_t)(c * 128));
+                    }
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     tmem_ld_touch(acc);
                     if (s == 2 * sh + 1) {
@@ -301,20 +306,19 @@ gcg_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ C
                         __syncwarp();
                         if (lane == 0) mbar_arrive(d_empty(dbuf));
                     }
+                    uint32_t yr[CH / 2];
 #pragma unroll
                     for (int c = 0; c < CH; c += 2) {
-                        // (16 s + c) & 7 == c & 7: the swizzle term of a column does not depend on the stream
-                        const uint32_t o0 = (uint32_t)((s * CH + c) * 128) + xo[c & 7], o1 = (uint32_t)((s * CH + c + 1) * 128) + xo[(c + 1) & 7];
                         f32x2 z = pk2(__uint_as_float(acc[c]), __uint_as_float(acc[c + 1]));
-                        if (a.bias_mode == VTX_BIAS_GATED) {
-                            const f32x2 kvv = pk2(__uint_as_float(lds16(kv_u + o0) << 16), __uint_as_float(lds16(kv_u + o1) << 16));
+                        if (skip) {
+                            const f32x2 kv2 = pk2(__uint_as_float(kvv[c] << 16), __uint_as_float(kvv[c + 1] << 16));
                             const f32x2 dd = *reinterpret_cast<const f32x2*>(dsk + c);
                             if (a.taps == VTX_TAPS_CONV) {
-                                z = fma2(dd, kvv, z);                       // fp32 sum, one rounding (engine.py:78,187)
+                                z = fma2(dd, kv2, z);                       // fp32 sum, one rounding (engine.py:78,187)
                             } else {
                                 float z0, z1, b0, b1;
                                 up2(z, z0, z1);
-                                up2(mul2(dd, kvv), b0, b1);
+                                up2(mul2(dd, kv2), b0, b1);
                                 const uint32_t zr = pack_bf16(z0, z1), br = pack_bf16(b0, b1);
                                 z = add2(pk2(bf_lo(zr), bf_hi(zr)), pk2(bf_lo(br), bf_hi(br)));
                             }
@@ -322,21 +326,47 @@ gcg_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ C
                         float z0, z1;
                         up2(z, z0, z1);
                         const uint32_t zr = pack_bf16(z0, z1);                 // the filter output in the I/O dtype
-                        const f32x2 qv = pk2(__uint_as_float(lds16(q_u + o0) << 16), __uint_as_float(lds16(q_u + o1) << 16));
+                        const f32x2 q2 = pk2(__uint_as_float(qv[c] << 16), __uint_as_float(qv[c + 1] << 16));
                         float y0, y1;
-                        up2(mul2(qv, pk2(bf_lo(zr), bf_hi(zr))), y0, y1);
-                        const uint32_t yr = pack_bf16(y0, y1);
-                        asm volatile("st.shared.u16 [%0], %1;" ::"r"(q_u + o0), "h"((unsigned short)(yr & 0xffffu)) : "memory");
-                        asm volatile("st.shared.u16 [%0], %1;" ::"r"(q_u + o1), "h"((unsigned short)(yr >> 16)) : "memory");
+                        up2(mul2(q2, pk2(bf_lo(zr), bf_hi(zr))), y0, y1);
+                        yr[c / 2] = pack_bf16(y0, y1);
+                    }
+#pragma unroll
+                    for (int c = 0; c < CH; c += 2) {
+                        asm volatile("st.shared.u16 [%0], %1;" ::"r"(qs_u + xo[c & 7] + (uint32_t)(c * 128)), "h"((unsigned short)(yr[c / 2] & 0xffffu)) : "memory");
+                        asm volatile("st.shared.u16 [%0], %1;" ::"r"(qs_u + xo[(c + 1) & 7] + (uint32_t)((c + 1) * 128)), "h"((unsigned short)(yr[c / 2] >> 16)) : "memory");
                     }
                 }
                 // k*v has been read: the slot may go; the tile of outputs goes to the TMA unit once all four warps wrote it
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) { mbar_arrive(kv_free(slot)); mbar_arrive(y_ready(oc & 1)); }
-                if (warp == W_EP && lane == 0 && mbar_wait(y_ready(oc & 1), (oc >> 1) & 1u, 42)) {
+                if (lane == 0) { mbar_arrive(kv_free(slot)); mbar_arrive(y_ready(qs)); }
+                if (sh == 0 && k == 1 && t + 1 < nmine && !expand(t + 1)) { ok = false; break; }
+            }
+        }
+    } else if (warp == W_ST) {
+        if (lane == 0) {
+            // ======== stores: a warp of their own.  Issuing a box takes a thread ~300 cycles, two to eight of them per chunk,
+            // and in an epilogue warp that held up the accumulator and the k*v slot of the whole CTA. ===================
+            int pending = -1;          // q stage whose tile of outputs the TMA unit may still be reading
+            bool ok = true;
+            for (int t = 0; t < nmine && ok; ++t) {
+                const int blk = item_blk(t);
+                // boxes of [16 channels x 64 samples] (x 4 batch elements) stored with whole 128-byte rows along time; samples
+                // past the end of the sequence are clipped by the tensor map
+                int x0[NS], bi[NS];
+                bool act[NS];
+#pragma unroll
+                for (int s = 0; s < NS; ++s) {
+                    const Stream st = stream_of(a, item_quad(t), s);
+                    x0[s] = (int)st.ts; bi[s] = (int)st.b; act[s] = st.active;
+                }
+                const int64_t d0 = (int64_t)blk * CH;
+                const int row = (int)(d0 % a.hdy), head = (int)(d0 / a.hdy);
+                for (int k = 1; k < nchunk; ++k, ++oc) {
+                    const int qs = oc % NQ;
+                    if (!mbar_wait(y_ready(qs), (oc / NQ) & 1u, 42)) { ok = false; break; }
                     const uint32_t src = sm_u + OFF_Q + qs * TILE;
-                    const int row = (int)(d0 % a.hdy), head = (int)(d0 / a.hdy);
 #pragma unroll
                     for (int hf = 0; hf < 2; ++hf) {
                         if (a.batch_quads) {
@@ -356,10 +386,7 @@ gcg_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ C
                     if (pending >= 0) mbar_arrive(q_empty(pending));
                     pending = qs;
                 }
-                if (sh == 0 && k == 1 && t + 1 < nmine && !expand(t + 1)) { ok = false; break; }
             }
-        }
-        if (warp == W_EP && lane == 0) {
             asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
             if (pending >= 0) mbar_arrive(q_empty(pending));
             asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");        // the last stores have landed before the CTA ends
