@@ -15,6 +15,8 @@
 // Precision.  g2 and z are products of two bf16 numbers: 16 significant bits, so head + remainder in bf16 hold them EXACTLY
 // (the fp32 kernels of gcg_bwd.cu work on the same exact products).  Taps are bf16, accumulation is fp32, one rounding on
 // the way out.  dw takes all four products of heads and remainders.
+// An infinite or NaN product makes its channel's dz NaN over the 256 rows of the contraction's window, not only under the
+// filter's taps (a zero tap times infinity), as in the forward kernel.
 //
 // What bounds it: 10 bytes in and 6 bytes out per element (B=2, L=8192, D=4096: 1.07 GB = 164 us at 6.54 TB/s), i.e. 2900
 // cycles per chunk and SM, of which the tensor pipe needs 16 x 85 (dz) + 8 x 128 (dw) and shared memory about as many.
