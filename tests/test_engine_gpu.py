@@ -278,6 +278,25 @@ def test_training_forward_saves_the_filter_output(bs, l, g, dg, hl):
     assert out.requires_grad and torch.equal(out.detach().nan_to_num(7.), want.nan_to_num(7.))
 
 
+@pytest.mark.parametrize("io", ["bf16", "f32"])       # the one-launch training forward, and the general one
+def test_training_forward_output_can_be_modified_in_place(io):
+    """A residual added in place to the operator's result (``y += r``): same gradients as the sum out of place."""
+    from vortex_b200 import hyena_ops
+
+    gen = torch.Generator().manual_seed(21)
+    ts = [torch.randn(2, 130, 2, 16, generator=gen).to(DT[io]).cuda().requires_grad_() for _ in range(3)]
+    h = (torch.randn(2, 1, 7, generator=gen) / 7 ** 0.5).to(DT[io]).cuda().requires_grad_()
+    r, dy = (torch.randn(2, 130, 2, 16, generator=gen).to(DT[io]).cuda() for _ in range(2))
+    y = hyena_ops.two_pass_chunked_gate_conv_gate(*ts, h)
+    want = y + r
+    grads = torch.autograd.grad(want, (*ts, h), dy)
+    y = hyena_ops.two_pass_chunked_gate_conv_gate(*ts, h)
+    y += r
+    assert torch.equal(y, want)
+    for a, b in zip(torch.autograd.grad(y, ts, dy), grads):
+        assert torch.equal(a, b)
+
+
 # ------------------------------------------------------------------ seeded parity against the oracle
 def _engine_block(eng, p, D, G, K, layout, ip=None, heads=1):
     """The reference's two-call sequence (model.py:233-291) on the drop-in engine."""

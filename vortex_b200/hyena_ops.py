@@ -273,11 +273,14 @@ class TwoPassChunkedGateConvGate(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, B, C, h):
+        bs, l, g, dg = x.shape
         if x.is_contiguous() and B.is_contiguous() and C.is_contiguous() and x.shape == B.shape == C.shape:
-            q3, k3, v3 = (t.view(*t.shape[:2], -1) for t in (C, B, x))
+            q3, k3, v3 = (t.view(bs, l, g * dg) for t in (C, B, x))
             if ops.gcg_cl_ok(q3, k3, v3, h):
-                # y and y2 from one launch: y2 rounded to bf16, y = C * y2 rounded again, as below
-                y, y2 = (t.view(x.shape) for t in ops.gcg_cl_fwd(q3, k3, v3, h, want_y2=True))
+                # y and y2 from one launch: y2 rounded to bf16, y = C * y2 rounded again, as below.  y is allocated in the
+                # shape it is returned in: a view made in here could not be modified in place by the caller
+                y, y2 = (torch.empty(x.shape, device=x.device, dtype=x.dtype) for _ in range(2))
+                ops.gcg_cl_fwd(q3, k3, v3, h, want_y2=True, out=(y.view(q3.shape), y2.view(q3.shape)))
                 ctx.save_for_backward(x, B, C, h, y2)
                 return y
         y2 = gcg_fwd(x, B, torch.ones_like(C), h)

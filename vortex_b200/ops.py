@@ -208,10 +208,12 @@ def gcg_cl_ok(q, k, v, h, bias_mode=BIAS_NONE) -> bool:
     return True
 
 
-def gcg_cl_fwd(q, k, v, h, bias=None, *, taps=TAPS_XCORR, bias_mode=BIAS_NONE, want_state=False, want_y2=False):
+def gcg_cl_fwd(q, k, v, h, bias=None, *, taps=TAPS_XCORR, bias_mode=BIAS_NONE, want_state=False, want_y2=False,
+               out=None):
     """Gate -> grouped FIR -> gate on channel-last operands q, k, v [B, L, D] (the hyena_ops layout with the group
     axes merged): one launch of the tensor-core kernel.  Returns y [B, L, D] and the inner cache [B, D, min(L, K-1)]
-    or None -- with ``want_y2`` the filter output before the gate [B, L, D] in the cache's place."""
+    or None -- with ``want_y2`` the filter output before the gate [B, L, D] in the cache's place.  ``out``: the
+    contiguous tensors (y, y2) to write instead of new ones."""
     _need_cuda(q, k, v, h, bias)
     B, L, D = q.shape
     h = _param(h, q)
@@ -219,7 +221,7 @@ def gcg_cl_fwd(q, k, v, h, bias=None, *, taps=TAPS_XCORR, bias_mode=BIAS_NONE, w
     h = h.reshape(G, -1)
     K = h.shape[1]
     bias = _param(bias, q)
-    y = torch.empty(B, L, D, device=q.device, dtype=q.dtype)
+    y, y2 = out if out is not None else (torch.empty(B, L, D, device=q.device, dtype=q.dtype), None)
     ns = min(L, K - 1)
     state = torch.empty(B, D, ns, device=q.device, dtype=q.dtype) if want_state else None
     p = _lib.GcgClParams(
@@ -230,7 +232,7 @@ def gcg_cl_fwd(q, k, v, h, bias=None, *, taps=TAPS_XCORR, bias_mode=BIAS_NONE, w
         bias_mode=bias_mode if bias is not None else BIAS_NONE, io_dtype=_code(q))
     with _on(q):
         if want_y2:
-            y2 = torch.empty_like(y)
+            y2 = torch.empty_like(y) if y2 is None else y2
             _lib.check(_lib.lib().vtx_gcg_cl_fwd_saving(C.byref(p), _ptr(y2), _stream(q)))
             return y, y2
         _lib.check(_lib.lib().vtx_gcg_cl_fwd(C.byref(p), _stream(q)))
