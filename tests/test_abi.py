@@ -86,6 +86,18 @@ def test_fused_iir_scratch_plan():
     assert q(1, 40, 4096, 4096) == 0                        # too short to cut
 
 
+@pytest.mark.parametrize("B,D,S,cplx", [(1, 4096, 16, 0), (1, 2048, 16, 0), (3, 768, 5, 1), (64, 4096, 16, 0), (2, 33, 16, 1),
+                                        (1, 1, 1, 0)])
+def test_long_conv_scratch_never_falls_with_the_length(B, D, S, cplx):
+    """A host sizes one carry buffer for its longest sequence and uses it for shorter ones; vtx_iir_fwd cannot see its size."""
+    f = _lib.lib().vtx_iir_scratch_bytes
+    most = 0
+    for L in list(range(1, 9000)) + list(range(9000, 140000, 977)):
+        n = f(B, L, D, S, cplx)
+        assert n >= most and n % (4 * B * D * S) == 0, L
+        most = n
+
+
 def test_conv_extension_argument_checks():
     """The conv extension's entry points report bad arguments by code before any launch, and the host wrappers
     reject CPU tensors, unknown activations and wrong layouts."""

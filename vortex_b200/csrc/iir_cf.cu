@@ -36,9 +36,13 @@ struct IirPlan {
 
 // Scratch a caller of vtx_iir_fwd has always been asked for, and the limit vtx_iir_fwd_noalloc has always refused by: the
 // carries of power-of-two segments of at least 512 samples, up to 1024 threads per SM.
-static int64_t iir_classic_segments(int64_t B, int64_t L, int64_t D) {
+static int64_t iir_classic_cuts(int64_t B, int64_t L, int64_t D) {
     int64_t nseg = 1;
     while (B * D * nseg < (int64_t)kNumSMs * 1024 && L / (nseg * 2) >= 512) nseg *= 2;
+    return nseg;
+}
+static int64_t iir_classic_segments(int64_t B, int64_t L, int64_t D) {
+    const int64_t nseg = iir_classic_cuts(B, L, D);
     const int64_t seg = ((L + nseg - 1) / nseg + 15) / 16 * 16;
     return (L + seg - 1) / seg;
 }
@@ -50,11 +54,16 @@ static int64_t iir_carry_bytes(int64_t B, int64_t D, int64_t nseg, int64_t S, bo
 // issue cycles in phase C and 22 more in phase A, and one block of four warps leaves its scheduler waiting for itself
 // about a third of the time.  At most four blocks per SM: more only add carries.  (L=4001, D=4096: 9 segments, two blocks
 // per SM, 98 us; 14 segments, which are 4 blocks too many for one round: 116 us.)
+static int64_t iir_most_segments(int64_t B, int64_t L, int64_t D) {
+    const int64_t by_blocks = (int64_t)kNumSMs * 4 * (ITHREADS / 32) / (B * ceil_div<int64_t>(D, 32)), by_length = L / (2 * ITT);
+    const int64_t n = by_blocks < by_length ? by_blocks : by_length;
+    return n > 1 ? n : 1;
+}
 static IirPlan iir_plan(int64_t B, int64_t L, int64_t D) {
-    const int64_t warps = B * ceil_div<int64_t>(D, 32);
+    const int64_t warps = B * ceil_div<int64_t>(D, 32), most = iir_most_segments(B, L, D);
     IirPlan best{1, ceil_div<int64_t>(L, ITT) * ITT};
     int64_t best_cost = INT64_MAX;
-    for (int64_t n = 1; n == 1 || (n <= L / (2 * ITT) && ceil_div<int64_t>(warps * n, ITHREADS / 32) <= (int64_t)kNumSMs * 4); ++n) {
+    for (int64_t n = 1; n <= most; ++n) {
         const int64_t seg = ceil_div<int64_t>(ceil_div<int64_t>(L, n), ITT) * ITT, nseg = ceil_div<int64_t>(L, seg);
         const int64_t per_sm = ceil_div<int64_t>(ceil_div<int64_t>(warps * nseg, ITHREADS / 32), kNumSMs);
         const int64_t cost = seg * (per_sm == 1 ? 3 : 2 * per_sm) * (nseg > 1 ? 77 : 55);
@@ -359,9 +368,10 @@ extern "C" int vtx_modal_filter(const vtx_modal_params* m, float* h, int64_t L, 
 extern "C" int64_t vtx_iir_scratch_bytes(int64_t B, int64_t L, int64_t D, int64_t S, int64_t complex_poles) {
     using namespace vtx;
     if (B <= 0 || L <= 0 || D <= 0 || S <= 0) return 0;
-    const int64_t now = iir_carry_bytes(B, D, iir_plan(B, L, D).nseg, S, complex_poles != 0);
-    const int64_t classic = iir_carry_bytes(B, D, iir_classic_segments(B, L, D), S, complex_poles != 0);
-    return now > classic ? now : classic;
+    // The most segments a plan may have, not those it does have after rounding (D=4096: 14 at L=1156, 9 at L=4096): the
+    // bytes never fall as L grows, so that a buffer sized for the longest sequence serves every shorter one.
+    const int64_t now = iir_most_segments(B, L, D), classic = iir_classic_cuts(B, L, D);
+    return iir_carry_bytes(B, D, now > classic ? now : classic, S, complex_poles != 0);
 }
 
 extern "C" int vtx_iir_fwd(const vtx_iir_params* p, void* stream) {
