@@ -287,8 +287,9 @@ int vtx_iir_recurrence_fwd(const vtx_iir_params* p, void* stream);
  * module loading the array's bytes are reserved on a device when the library's long-convolution module is first
  * used there (this first call, or the first vtx_iir_fwd / vtx_modal_filter), not when the library is loaded: make
  * that call during start-up, BEFORE the host hands the rest of the device memory to its own pools, or the
- * reservation itself can fail with an out-of-memory launch error.  All calls share the
- * array and it keeps the last call's contents (nothing needs clearing); calls that overlap on the GPU race.
+ * reservation itself can fail with an out-of-memory launch error.  Calls of L < 1024, or of B * D >= 148 * 1024, do
+ * not touch the array.  All others share it and it keeps the last call's contents (nothing needs clearing); those
+ * race when they overlap on the GPU.
  * Calls no cudaMalloc, cudaFree or other allocating routine. */
 #define VTX_IIR_STATIC_SCRATCH_BYTES (16u << 20)
 int vtx_iir_fwd_noalloc(const vtx_iir_params* p, void* stream);

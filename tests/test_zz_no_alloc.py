@@ -33,6 +33,27 @@ def test_noalloc_entry_point_matches_scratch_entry_point_twice():
         assert torch.equal(st, st_ref), f"call {call}: states differ"
 
 
+def test_noalloc_leaves_the_shared_array_alone_at_short_lengths():
+    """Below 1024 samples a row is one segment and the shared array is not touched, so that such calls may overlap on
+    the GPU: one launch (three where carries pass through the array), the result of the call with a buffer of its own."""
+    from helpers import TOL, check, rel_l2
+    from vortex_b200 import ops
+
+    B, D, S = 2, 64, 16
+    g = torch.Generator().manual_seed(5)
+    log_poles = torch.log(0.9 + 0.099 * torch.rand(D, S, generator=g)).cuda()
+    residues, bias = torch.randn(D, S, generator=g).cuda(), torch.randn(D, generator=g).bfloat16().cuda()
+    for L, launches in ((1023, 1), (1024, 3)):
+        z = torch.randn(B, 3 * D, L, generator=g).bfloat16().cuda()
+        y_ref, st_ref = ops.iir_fwd(z, log_poles, residues, bias, D)
+        y, st = torch.empty(B, D, L, dtype=z.dtype, device="cuda"), torch.empty_like(st_ref)
+        before = ops.launch_count()
+        ops.iir_fwd_noalloc(z, log_poles, residues, bias, D, y, st)
+        assert ops.launch_count() - before == launches, L
+        check(f"long convolution without a buffer, L={L}", rel_l2(y, y_ref), TOL["bf16"])
+        check(f"its state, L={L}", rel_l2(st, st_ref), 2e-5)
+
+
 def test_noalloc_entry_point_refuses_sizes_beyond_its_scratch():
     from vortex_b200 import _lib, ops
 

@@ -454,9 +454,9 @@ extern "C" int vtx_iir_recurrence_fwd(const vtx_iir_params* p, void* stream) {
 //   commits the rest of the device memory: with CUDA's default lazy module loading the array is reserved on a
 //   device when this file's module is first used there (this call, vtx_iir_fwd or vtx_modal_filter), not when
 //   the library is loaded.
-// * All calls share the one array and it keeps whatever the last call left in it.  Nothing in it has to be
-//   zero at the start: every word a call reads was written earlier by the same call, except the carry slot of
-//   the last segment, whose value is computed but never used.  Two calls that overlap on the GPU (different
+// * Calls of L < 1024, or of 148 * 1024 rows and more, do not touch the array (one segment per row).  All others
+//   share it, and it keeps whatever the last of them left in it.  Nothing in it has to be zero at the start: every
+//   word a call reads was written earlier by the same call.  Two of these that overlap on the GPU (different
 //   streams, or different host threads) race on the array: serialise them.
 // * No cudaMalloc / cudaFree / allocating library routine is called on this path.
 constexpr size_t kIirStaticScratchBytes = VTX_IIR_STATIC_SCRATCH_BYTES;
@@ -485,6 +485,7 @@ extern "C" int vtx_iir_fwd_noalloc(const vtx_iir_params* p, void* stream) {
         dev_ptr[dev] = ptr;
     }
     vtx_iir_params q = *p;
-    q.scratch = dev_ptr[dev];
+    // one segment per row where vtx_iir_fwd accepts no scratch: such calls may overlap
+    q.scratch = iir_classic_segments(p->B, p->L, p->D) == 1 ? nullptr : dev_ptr[dev];
     return vtx_iir_fwd(&q, stream);
 }

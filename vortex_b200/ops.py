@@ -569,7 +569,8 @@ def iir_fwd_noalloc(z_pre: torch.Tensor, log_poles, residues, bias, D: int, y: t
     Nothing is allocated here or in the library: ``y`` [B, D, L] (dtype of ``z_pre``) and ``state`` (fp32
     [B, D, S] or [B, D, S, 2], or None) are the caller's, the parameters must already be fp32, contiguous and
     on the device, and the segment carries go into the scratch array built into the library.  Sizes beyond
-    that array raise NotImplementedError.  Calls share the array: do not overlap them on the GPU."""
+    that array raise NotImplementedError.  Calls of 1024 samples and more share the array: do not overlap them on the
+    GPU."""
     _need_cuda(z_pre, residues, log_poles, bias, y, state)
     B, C3, L = z_pre.shape
     if C3 != 3 * D or z_pre.stride(2) != 1:
