@@ -249,7 +249,8 @@ int vtx_modal_filter(const vtx_modal_params* m, float* h, int64_t L, void* strea
  * (engine.py:262-353,404) and prefill_via_modal_fft (engine.py:525-559).
  *   y [B,D,L] (strided: the engine returns it viewed as [B,L,D]);
  *   state fp32 [B,D,S] (real poles) or [B,D,S,2] (complex), or NULL.
- * scratch: fp32, vtx_iir_scratch_bytes(...) bytes, may be NULL when that is 0.  The bytes never fall as L grows
+ * scratch: fp32, vtx_iir_scratch_bytes(...) bytes; may be NULL when that is 0, when L < 1024 and when
+ *   B * D >= 148 * 1024 (a row is then one segment; with a buffer it may be cut, which is faster).  The bytes never fall as L grows
  *   with the other sizes fixed: a buffer sized for the longest sequence serves every shorter one.
  * ------------------------------------------------------------------------ */
 typedef struct vtx_iir_params {

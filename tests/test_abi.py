@@ -98,6 +98,14 @@ def test_long_conv_scratch_never_falls_with_the_length(B, D, S, cplx):
         most = n
 
 
+@pytest.mark.parametrize("B,L,D", [(1, 1024, 64), (1, 131072, 4096), (37, 4096, 4095)])
+def test_long_conv_without_scratch_is_refused_where_it_is_needed(B, L, D):
+    """(The sizes that need none run on a GPU: test_engine_gpu.py.)"""
+    p = _lib.IirParams(q=16, k=16, v=16, y=16, B=B, L=L, D=D, head_dim=D)
+    p.modal.G, p.modal.S, p.modal.log_poles, p.modal.res_re = D, 16, 16, 16
+    assert _lib.lib().vtx_iir_fwd(C.byref(p), None) == -1 and "scratch needed" in _lib.last_error()
+
+
 def test_conv_extension_argument_checks():
     """The conv extension's entry points report bad arguments by code before any launch, and the host wrappers
     reject CPU tensors, unknown activations and wrong layouts."""

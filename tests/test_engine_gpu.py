@@ -491,6 +491,25 @@ def test_long_conv_tiles(io, B, L, D, G, S, cplx, layout, heads):
     assert torch.equal(y, outs[1][0]) and torch.equal(st, outs[1][1])
 
 
+@pytest.mark.parametrize("B,L,D", [(1, 1, 33), (2, 65, 64), (1, 1023, 96), (38, 1030, 4000)])
+def test_long_conv_without_scratch(monkeypatch, B, L, D):
+    """A NULL buffer at the sizes that need none (L < 1024, or rows for every thread of the GPU): one launch, and the
+    result of the call with a buffer."""
+    from vortex_b200 import _lib, ops
+
+    g = torch.Generator(device="cuda").manual_seed(2)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    z, bias, res = r(B, 3 * D, L).bfloat16(), r(D).bfloat16(), r(D, 16)
+    lp = torch.log(0.9 + 0.099 * torch.rand(D, 16, device="cuda", generator=g))
+    y, st = ops.iir_fwd(z, lp, res, bias, D)
+    monkeypatch.setattr(_lib.lib(), "vtx_iir_scratch_bytes", lambda *a: 0)
+    before = ops.launch_count()
+    y0, st0 = ops.iir_fwd(z, lp, res, bias, D)
+    assert ops.launch_count() - before == 1
+    check(f"long convolution without scratch L={L} y", rel_l2(y0, y), TOL["bf16"])
+    check(f"long convolution without scratch L={L} state", rel_l2(st0, st), 2e-5)
+
+
 @pytest.mark.parametrize("io,L,kind", [("bf16", 4001, "mr"), ("bf16", 129, "se"), ("f16", 1003, "se"), ("bf16", 127, "mr")])
 def test_rows_of_an_odd_length(eng, io, L, kind):
     """The drop-in calls on lengths whose rows need padding to start on 16-byte boundaries: identical to the same calls on

@@ -386,7 +386,7 @@ extern "C" int vtx_iir_fwd(const vtx_iir_params* p, void* stream) {
     IirPlan pl = iir_plan(p->B, p->L, p->D);
     VTX_REQUIRE(iir_classic_segments(p->B, p->L, p->D) == 1 || p->scratch, VTX_ERR_BAD_ARG, "iir: scratch needed (%lld bytes)",
                 (long long)vtx_iir_scratch_bytes(p->B, p->L, p->D, p->modal.S, cplx));
-    if (!p->scratch) pl = IirPlan{1, ceil_div<int64_t>(p->L, ITT) * ITT};      // sizes that were never asked for any
+    if (!p->scratch) pl = IirPlan{1, ceil_div<int64_t>(p->L, ITT) * ITT};      // sizes that need none
     cudaStream_t s = (cudaStream_t)stream;
     const int64_t es = dtype_size(p->io_dtype);
     auto al = [&](const void* q, int64_t s0, int64_t s1, int64_t s2) {
