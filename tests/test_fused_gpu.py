@@ -688,6 +688,39 @@ def test_prefill_caches_of_walks_with_several_items():
 
 
 @pytest.mark.gpu
+def test_native_host_calls_do_not_hold_the_gil():
+    """The C++ argument handling calls the library, and allocates, without the GIL.  The interpreter's own
+    PyGILState_Check stands in for the library's functions: 0 (a success status) without the GIL, 1 (an error) with it.
+    Errors are still raised as they are."""
+    import ctypes
+
+    from vortex_b200 import _lib, ops
+
+    D = 32
+    z = lambda *s: torch.zeros(*s, device="cuda")  # noqa: E731
+    calls = [lambda: ops.decode_layer(z(1, 3 * D), z(3 * D, 1, 3), None, z(1, 3 * D, 2), D, h=z(2, 1, 7), inner_state=z(1, D, 6)),
+             lambda: ops.fused_fir_fwd(z(1, 8, 3 * D), z(3 * D, 1, 3), None, z(2, 1, 7), None, D, taps=_lib.TAPS_XCORR,
+                                       bias_mode=_lib.BIAS_NONE),
+             lambda: ops.fused_iir_fwd(z(1, 8, 3 * D), z(3 * D, 1, 3), z(D, 16), z(D, 16), z(D), D)]
+    addr = lambda f: ctypes.cast(f, ctypes.c_void_p).value  # noqa: E731
+    real = [addr(getattr(_lib.lib(), "vtx_" + n)) for n in ("decode_layer", "fused_fir_fwd", "fused_iir_fwd", "fused_iir_scratch_bytes",
+                                                            "last_error")]
+    host = _lib.host()
+    try:
+        host.bind(*[addr(ctypes.pythonapi.PyGILState_Check)] * 3, *real[3:])
+        for f in calls:
+            f()
+    finally:
+        host.bind(*real)
+    for f in calls:
+        f()
+    with pytest.raises(ValueError, match="packed channels"):
+        ops.decode_layer(z(1, D), z(3 * D, 1, 3), None, z(1, 3 * D, 2), D, h=z(2, 1, 7), inner_state=z(1, D, 6))
+    with pytest.raises(NotImplementedError, match="full inner cache"):
+        ops.decode_layer(z(1, 3 * D), z(3 * D, 1, 3), None, z(1, 3 * D, 2), D, h=z(2, 1, 7), inner_state=z(1, D, 5))
+
+
+@pytest.mark.gpu
 def test_fused_mr_call_cut_into_launches():
     """A call large enough to be cut into several launches (24 sequences of 8192 tokens, 4096 channels: 6.4 GB moved)
     gives, bit for bit, what single-launch calls on slices of the batch give, caches included; the oracle agrees on a

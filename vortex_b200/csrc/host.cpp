@@ -22,7 +22,9 @@ decltype(&vtx_fused_iir_fwd) p_fused_iir_fwd;
 decltype(&vtx_fused_iir_scratch_bytes) p_fused_iir_scratch_bytes;
 decltype(&vtx_last_error) p_last_error;
 
+// The entry points run without the GIL (see the module definition); an error is made with it.
 [[noreturn]] void raise(PyObject* type, const std::string& msg) {
+    const py::gil_scoped_acquire gil;
     PyErr_SetString(type, msg.c_str());
     throw py::error_already_set();
 }
@@ -253,7 +255,9 @@ PYBIND11_MODULE(_vtx_host, m) {
         p_fused_iir_scratch_bytes = reinterpret_cast<decltype(p_fused_iir_scratch_bytes)>(iir_scratch);
         p_last_error = reinterpret_cast<decltype(p_last_error)>(last_error);
     });
-    m.def("decode_layer", &decode_layer);
-    m.def("fused_fir_fwd", &fused_fir_fwd);
-    m.def("fused_iir_fwd", &fused_iir_fwd);
+    // Without the GIL, as torch's own calls and calls through ctypes are: an allocation or a launch into a full queue can
+    // block, and the process's other threads go on meanwhile.
+    m.def("decode_layer", &decode_layer, py::call_guard<py::gil_scoped_release>());
+    m.def("fused_fir_fwd", &fused_fir_fwd, py::call_guard<py::gil_scoped_release>());
+    m.def("fused_iir_fwd", &fused_iir_fwd, py::call_guard<py::gil_scoped_release>());
 }
