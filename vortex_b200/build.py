@@ -1,7 +1,8 @@
 """Builds ``vortex_b200/lib/libvortex_b200.so`` from ``vortex_b200/csrc/*.cu`` with nvcc for sm_100a, and the host
-module ``vortex_b200/lib/_vtx_host.so`` from ``csrc/host.cpp`` with g++ against torch's headers.
+module ``vortex_b200/lib/_vtx_host.so`` from ``csrc/host.cpp`` with g++ against torch's and Python's headers.
 
     python -m vortex_b200.build [--force] [--verbose]
+    python vortex_b200/build.py          # the same where torch is not installed: the library (C ABI) alone
 
 nvcc cross-compiles without a GPU.  Objects are rebuilt only when their source (or a header)
 changed.  The library is kept in-tree so that it travels with the checkout.
@@ -72,7 +73,11 @@ def _compile(src: str, force: bool, verbose: bool) -> tuple[str, bool, str]:
 def _build_host(force: bool) -> None:
     import sysconfig
 
-    import torch
+    try:
+        import torch
+    except ImportError:          # the module serves the Python wrappers, which need torch; the C ABI does not
+        print("torch not found: host module not built", file=sys.stderr)
+        return
     from torch.utils import cpp_extension as ext
 
     stamp = os.path.join(OBJDIR, "host.sha")
@@ -82,8 +87,8 @@ def _build_host(force: bool) -> None:
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     libdir = os.path.join(os.path.dirname(torch.__file__), "lib")
     inc = [*ext.include_paths(), os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
-    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-w", "-DTORCH_API_INCLUDE_EXTENSION_H",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{d}" for d in inc), HOST_SRC,
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-Wall", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-isystem{d}" for d in inc), HOST_SRC,
            "-o", HOST_LIB, f"-L{libdir}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
@@ -98,17 +103,19 @@ def build(force: bool = False, verbose: bool = False) -> str:
     with cf.ThreadPoolExecutor(max_workers=min(8, len(srcs)) + 1) as ex:
         host = ex.submit(_build_host, force)
         results = list(ex.map(lambda s: _compile(s, force, verbose), srcs))
-        host.result()
     objs = [o for o, _, _ in results]
     if verbose:
         for _, _, log in results:
             if log:
                 print(log, file=sys.stderr)
-    if any(changed for _, changed, _ in results) or not os.path.exists(LIB):
+    # (an object newer than the library: an earlier build ended between the two)
+    if any(changed for _, changed, _ in results) or not os.path.exists(LIB) or \
+            max(map(os.path.getmtime, objs)) > os.path.getmtime(LIB):
         cmd = [_nvcc(), "-shared", "-o", LIB] + objs + ["-gencode", "arch=compute_100a,code=sm_100a"]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    host.result()                # (raises what the host module's build raised, the library being linked)
     return LIB
 
 
