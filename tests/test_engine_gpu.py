@@ -510,6 +510,20 @@ def test_long_conv_without_scratch(monkeypatch, B, L, D):
     check(f"long convolution without scratch L={L} state", rel_l2(st0, st), 2e-5)
 
 
+@pytest.mark.parametrize("L", [1000, 1003])       # the kernel with tensor maps takes both, z's rows being padded
+def test_featurizer_batch_pitches(L):
+    """Batch pitches that no tensor map can hold: a single sequence whose (unused) pitch is odd, a batch expanded from one
+    sequence.  Same z and cache as on a contiguous copy, bit for bit."""
+    from vortex_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(8)
+    u = torch.randn(1, L, 96, device="cuda", generator=g).bfloat16()
+    w = torch.randn(96, 1, 3, device="cuda", generator=g).bfloat16()
+    for v in (u.as_strided((1, L, 96), (5, 96, 1)), u.expand(3, -1, -1)):
+        for a, b in zip(ops.featurizer_fwd(v, w), ops.featurizer_fwd(v.clone(memory_format=torch.contiguous_format), w)):
+            assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("io,L,kind", [("bf16", 4001, "mr"), ("bf16", 129, "se"), ("f16", 1003, "se"), ("bf16", 127, "mr")])
 def test_rows_of_an_odd_length(eng, io, L, kind):
     """The drop-in calls on lengths whose rows need padding to start on 16-byte boundaries: identical to the same calls on

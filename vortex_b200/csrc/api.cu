@@ -57,6 +57,7 @@ int make_tmap_3d(CUtensorMap* out, const void* base, int64_t dtype, int64_t cols
     EncodeTiledFn fn = encode_fn();
     if (!fn) return fail(VTX_ERR_LAUNCH, "%s: cuTensorMapEncodeTiled entry point unavailable", who);
     const int64_t es = dtype_size(dtype);
+    if (batch == 1) batch_stride = row_stride * rows;      // never stepped: any legal pitch
     if (reinterpret_cast<uintptr_t>(base) % 16 || (row_stride * es) % 16 || (batch_stride * es) % 16)
         return fail(VTX_ERR_ALIGNMENT, "%s: base address and row/batch pitch must be multiples of 16 bytes", who);
     if ((box_cols * es) % 16) return fail(VTX_ERR_ALIGNMENT, "%s: box width must be a multiple of 16 bytes", who);
@@ -65,7 +66,6 @@ int make_tmap_3d(CUtensorMap* out, const void* base, int64_t dtype, int64_t cols
                                                  : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batch};
     cuuint64_t strides[2] = {(cuuint64_t)(row_stride * es), (cuuint64_t)(batch_stride * es)};
-    if (batch == 1) strides[1] = strides[0] * (cuuint64_t)rows;   // any legal value: never used to step
     cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1};
     cuuint32_t estr[3] = {1, 1, 1};
     CUtensorMapSwizzle sw = swizzle_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B

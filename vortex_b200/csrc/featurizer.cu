@@ -225,8 +225,9 @@ extern "C" int vtx_featurizer_fwd_pitched(const vtx_featurizer_params* p, int64_
     VTX_REQUIRE(valid_dtype(p->w_dtype) && (!p->bias || valid_dtype(p->bias_dtype)) &&
                     (!p->mask || valid_dtype(p->mask_dtype)),
                 VTX_ERR_BAD_ARG, "featurizer: bad parameter dtype");
+    // (a tensor map steps by positive pitches: a batch expanded from one sequence takes the general kernel)
     const bool tma_ok = p->io_dtype != VTX_F32 && p->u_stride_c == 1 && reinterpret_cast<uintptr_t>(p->u) % 16 == 0 &&
-                        p->u_stride_l % 8 == 0 && (p->B == 1 || p->u_stride_b % 8 == 0) && p->u_stride_l > 0 &&
+                        p->u_stride_l % 8 == 0 && (p->B == 1 || (p->u_stride_b > 0 && p->u_stride_b % 8 == 0)) && p->u_stride_l > 0 &&
                         reinterpret_cast<uintptr_t>(p->z) % 16 == 0 && pitch % 8 == 0 && pitch < ((int64_t)1 << 31) - 256 &&
                         p->C < ((int64_t)1 << 31) && ceil_div<int64_t>(p->L, FTT) <= 65535;
     if (tma_ok) {
