@@ -545,6 +545,37 @@ def test_rows_of_an_odd_length(eng, io, L, kind):
     check(f"gate-conv-gate {kind} {io} L={L}", rel_l2(y, y2), TOL[io])
 
 
+@pytest.mark.parametrize("B,L,D,K", [(1, 1, 16, 7), (1, 129, 32, 128), (2, 4001, 48, 128), (3, 1003, 80, 7), (5, 263, 2400, 33)])
+def test_outputs_of_an_odd_length_are_dense(eng, B, L, D, K):
+    """The gate-conv-gate and long-filter outputs are contiguous at every length, also on the featurizer's padded rows:
+    ``.view`` works on them, and a call that wants a contiguous output buffer takes them.  The kernel that stores them
+    sample by sample writes what it writes by whole boxes at the next multiple of 8, bit for bit."""
+    from vortex_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(L)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    Lp = (L + 7) // 8 * 8
+    zp = torch.zeros(B, 3 * D, Lp, device="cuda", dtype=torch.bfloat16)
+    z = zp[..., :L]
+    z.copy_(r(B, 3 * D, L))
+    h, bias = (r(D // 16, 1, K) / K ** 0.5).bfloat16(), r(D).bfloat16()
+    kw = dict(dims=(D, 1, D, 16, D // 16), groups=D // 16, gated_bias=True, dim_last=False, fir_length=K, gate=True,
+              inference_params=True)
+    rows = h.repeat_interleave(16, 0)
+    y, st = eng.parallel_fir(F.conv1d, z, rows, bias, L, **kw)
+    assert y.view(B, D * L).shape == (B, D * L)
+    assert torch.equal(y, eng.parallel_fir(F.conv1d, zp, rows, bias, Lp, **kw)[0][..., :L])
+    assert torch.equal(st, eng.parallel_fir(F.conv1d, z.contiguous(), rows, bias, L, **kw)[1])
+    lp = torch.log(0.9 + 0.099 * torch.rand(D, 16, device="cuda", generator=g))
+    res = r(D, 16)
+    y, st = ops.iir_fwd(z, lp, res, bias, D)
+    assert y.view(B, D * L).shape == (B, D * L)
+    again = torch.zeros_like(y)
+    ops.iir_fwd_noalloc(z, lp, res, bias, D, y, None)
+    ops.iir_fwd_noalloc(z, lp, res, bias, D, again, None)
+    assert torch.equal(y, again)
+
+
 def test_padding_mask_and_errors(eng):
     B, L, D, G, K = 2, 40, 32, 2, 7
     p = cuda(make_block(21, B, L, D, G, K, "f32"))

@@ -71,6 +71,7 @@ struct Args {
     int64_t hdy;                           // "head" size of the output's tensor map (D: y has one channel pitch)
     int64_t nseg, seg_len, nquad, nitems, nblk;   // nblk = D / 16 channel blocks
     int taps, bias_mode, batch_quads;      // batch_quads: mode A
+    int y_plain;                           // y rows off the 16-byte boundaries: no tensor map for them
 };
 
 struct Stream {
@@ -345,7 +346,34 @@ gcg_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ C
             }
         }
     } else if (warp == W_ST) {
-        if (lane == 0) {
+        if (a.y_plain) {
+            // ======== stores of rows that no TMA box can hold: 64 bytes of a row at a time, sample by sample ==============
+            bool ok = true;
+            for (int t = 0; t < nmine && ok; ++t) {
+                const int64_t d0 = (int64_t)item_blk(t) * CH;
+                for (int k = 1; k < nchunk; ++k, ++oc) {
+                    const int qs = oc % NQ;
+                    if (!mbar_wait(y_ready(qs), (oc / NQ) & 1u, 45)) { ok = false; break; }
+#pragma unroll 1
+                    for (int s = 0; s < NS; ++s) {
+                        const Stream st = stream_of(a, item_quad(t), s);
+                        const int64_t x = st.ts + (k - 1) * CHUNK, left = st.active ? a.L - x : 0;
+                        unsigned short* const y = reinterpret_cast<unsigned short*>(a.y) + st.b * a.y_stride_b + d0 * a.y_stride_d + x;
+#pragma unroll 8
+                        for (int c = 0; c < CH; ++c)
+#pragma unroll
+                            for (int m = lane; m < CHUNK; m += 32)
+                                if (m < left) {
+                                    unsigned short v;
+                                    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(sm_u + OFF_Q + qs * TILE + tile_off(s * CH + c, m)));
+                                    y[c * a.y_stride_d + m] = v;
+                                }
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(q_empty(qs));
+                }
+            }
+        } else if (lane == 0) {
             // ======== stores: a warp of their own.  Issuing a box takes a thread ~300 cycles, two to eight of them per chunk,
             // and in an epilogue warp that held up the accumulator and the k*v slot of the whole CTA. ===================
             int pending = -1;          // q stage whose tile of outputs the TMA unit may still be reading
@@ -505,9 +533,7 @@ bool gcg_tc_shape(const vtx_gcg_params* p) {
         p->bias_mode == VTX_BIAS_ADD)
         return false;
     if (p->D % CH || p->G <= 0 || p->D % p->G || (p->D / p->G) % CH || p->head_dim % CH) return false;
-    if (p->y_stride_l != 1 || reinterpret_cast<uintptr_t>(p->y) % 16 || p->y_stride_d <= 0 || p->y_stride_d % 8 ||
-        (p->B > 1 && (p->y_stride_b <= 0 || p->y_stride_b % 8)))
-        return false;
+    if (p->y_stride_l != 1) return false;
     const void* ptrs[3] = {p->q, p->k, p->v};
     const int64_t sd[3] = {p->q_stride_d, p->k_stride_d, p->v_stride_d}, sh[3] = {p->q_stride_h, p->k_stride_h, p->v_stride_h},
                   sb[3] = {p->q_stride_b, p->k_stride_b, p->v_stride_b};
@@ -556,10 +582,14 @@ int gcg_tc_fwd(const vtx_gcg_params* p, cudaStream_t stream) {
         if (int rc = make_tmap_bhdl(&tm[i], ptrs[i], VTX_BF16, p->L, p->head_dim, p->D / p->head_dim, p->B, sd[i], sh[i], sb[i],
                                     64, CH, a.batch_quads ? NS : 1, "gcg(tensor cores)"))
             return rc;
-    CUtensorMap tmy;
-    if (int rc = make_tmap_bhdl(&tmy, p->y, VTX_BF16, p->L, p->D, 1, p->B, p->y_stride_d, p->y_stride_d * p->D, p->y_stride_b,
-                                64, CH, a.batch_quads ? NS : 1, "gcg(tensor cores, y)"))
-        return rc;
+    // y on 16-byte rows leaves by TMA; a dense y of an odd length (operands on padded rows) by plain stores
+    CUtensorMap tmy = tm[0];
+    a.y_plain = reinterpret_cast<uintptr_t>(p->y) % 16 || p->y_stride_d <= 0 || p->y_stride_d % 8 ||
+                (p->B > 1 && (p->y_stride_b <= 0 || p->y_stride_b % 8));
+    if (!a.y_plain)
+        if (int rc = make_tmap_bhdl(&tmy, p->y, VTX_BF16, p->L, p->D, 1, p->B, p->y_stride_d, p->y_stride_d * p->D, p->y_stride_b,
+                                    64, CH, a.batch_quads ? NS : 1, "gcg(tensor cores, y)"))
+            return rc;
     a.hdy = p->D;
     static bool attr_set[64] = {};
     static int resident[64] = {};

@@ -76,17 +76,13 @@ def launch_count() -> int:
     return int(_lib.lib().vtx_launch_count())
 
 
-def _rows(B: int, R: int, L: int, like: torch.Tensor, aligned: bool = True) -> torch.Tensor:
+def _rows(B: int, R: int, L: int, like: torch.Tensor) -> torch.Tensor:
     """Uninitialised [B, R, L] with every row on a 16-byte boundary: the first L samples of rows of whole 16-byte vectors
-    (a contiguous tensor where L is a multiple of them, or where ``aligned`` is false)."""
+    (a contiguous tensor where L is a multiple of them)."""
     n = 16 // like.element_size()
-    pitch = -(-L // n) * n if aligned else L
+    pitch = -(-L // n) * n
     t = torch.empty(B, R, pitch, device=like.device, dtype=like.dtype)
     return t if pitch == L else t[..., :L]
-
-
-def _rows_aligned(t: torch.Tensor, *strides: int) -> bool:
-    return t.data_ptr() % 16 == 0 and all(s * t.element_size() % 16 == 0 for s in strides)
 
 
 # ----------------------------------------------------------------------------------------------
@@ -162,9 +158,8 @@ def _gcg_raw(q, k, v, sb, sh, sd, hd, h, bias, B, L, D, *, taps, bias_mode, mask
         y = torch.empty(B, L, D, device=dev, dtype=dt)
         ysb, ysd, ysl = L * D, 1, D
     else:
-        # operands with 16-byte aligned rows: the outputs' rows are laid out alike
-        y = _rows(B, D, L, q, all(_rows_aligned(t, s) for t, s in zip((q, k, v), sd if isinstance(sd, tuple) else (sd,) * 3)))
-        ysb, ysd, ysl = y.stride(0), y.stride(1), 1
+        y = torch.empty(B, D, L, device=dev, dtype=dt)
+        ysb, ysd, ysl = D * L, L, 1
     ns = min(L, K - 1)
     state = torch.empty(B, D, ns, device=dev, dtype=dt) if want_state else None
     sbs = sb if isinstance(sb, tuple) else (sb, sb, sb)
@@ -440,7 +435,7 @@ def causal_conv1d_varlen_states(x: torch.Tensor, cu_seqlens: torch.Tensor, state
 
 def iir_fwd(z_pre: torch.Tensor, log_poles, residues, bias, D: int, *, layout="split", num_heads=1, flip=False,
             theta=None, res_im=None, want_state=True, round_kv=True):
-    """Gate -> modal long convolution -> gate.  z_pre [B, 3D, L] -> y [B, D, L] (rows aligned as z_pre's are), state fp32
+    """Gate -> modal long convolution -> gate.  z_pre [B, 3D, L] -> y [B, D, L] (contiguous), state fp32
     [B, D, S] (or [B, D, S, 2] for complex poles) or None."""
     _need_cuda(z_pre, residues, bias)
     if z_pre.stride(2) != 1:
@@ -452,7 +447,7 @@ def iir_fwd(z_pre: torch.Tensor, log_poles, residues, bias, D: int, *, layout="s
     m, keep = _modal(log_poles, residues, z_pre, theta, res_im)
     cplx = theta is not None
     bias = _param(bias, z_pre)
-    y = _rows(B, D, L, z_pre, _rows_aligned(z_pre, z_pre.stride(1)))
+    y = torch.empty(B, D, L, device=z_pre.device, dtype=z_pre.dtype)
     state = None
     if want_state:
         state = torch.empty((B, D, m.S, 2) if cplx else (B, D, m.S), device=z_pre.device, dtype=torch.float32)
@@ -463,7 +458,7 @@ def iir_fwd(z_pre: torch.Tensor, log_poles, residues, bias, D: int, *, layout="s
         k=_ptr(k), k_stride_b=z_pre.stride(0), k_stride_h=sh, k_stride_d=sd,
         v=_ptr(v), v_stride_b=z_pre.stride(0), v_stride_h=sh, v_stride_d=sd, head_dim=hd, modal=m,
         bias=_ptr(bias), bias_dtype=_code(bias) if bias is not None else 0,
-        y=_ptr(y), y_stride_b=y.stride(0), y_stride_d=y.stride(1), y_stride_l=1, state=_ptr(state), scratch=_ptr(scratch),
+        y=_ptr(y), y_stride_b=D * L, y_stride_d=L, y_stride_l=1, state=_ptr(state), scratch=_ptr(scratch),
         B=B, L=L, D=D, round_kv=int(round_kv), io_dtype=_code(z_pre))
     with _on(z_pre):
         _lib.check(_lib.lib().vtx_iir_fwd(C.byref(p), _stream(z_pre)))
