@@ -71,7 +71,6 @@ struct Args {
     int64_t hdy;                           // "head" size of the output's tensor map (D: y has one channel pitch)
     int64_t nseg, seg_len, nquad, nitems, nblk;   // nblk = D / 16 channel blocks
     int taps, bias_mode, batch_quads;      // batch_quads: mode A
-    int y_plain;                           // y rows off the 16-byte boundaries: no tensor map for them
 };
 
 struct Stream {
@@ -106,6 +105,8 @@ __device__ __forceinline__ uint32_t tile_off(int n, int t) {
     return (uint32_t)((t >> 6) * HALF_TILE + n * 128 + ((((t & 63) >> 3) ^ (n & 7)) << 4) + (t & 7) * 2);
 }
 
+// PLAIN: y's rows do not start on 16-byte boundaries, so no tensor map holds them
+template <bool PLAIN>
 __global__ void __launch_bounds__(THREADS, 1)
 gcg_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ CUtensorMap tmk,
               const __grid_constant__ CUtensorMap tmv, const __grid_constant__ CUtensorMap tmy,
@@ -332,6 +333,17 @@ gcg_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ C
                         up2(mul2(q2, pk2(bf_lo(zr), bf_hi(zr))), y0, y1);
                         yr[c / 2] = pack_bf16(y0, y1);
                     }
+                    if (PLAIN) {
+                        // 64 bytes of a row per warp and channel, the neighbouring warps' next to them (a warp of its own that
+                        // stored the tile's rows, sample by sample or in shifted vectors, took 85 and 115 us for the 61 at
+                        // B=1, L=4001, D=4096, 128 taps; whole boxes at L=4000 take 53)
+                        const Stream st = stream_of(a, item_quad(t), s);
+                        const int64_t x = st.ts + (k - 1) * CHUNK + r;
+                        unsigned short* y = reinterpret_cast<unsigned short*>(a.y) + st.b * a.y_stride_b + (int64_t)blk * CH * a.y_stride_d + x;
+                        if (st.active && x < a.L)
+#pragma unroll
+                            for (int c = 0; c < CH; ++c, y += a.y_stride_d) *y = (unsigned short)(c & 1 ? yr[c / 2] >> 16 : yr[c / 2] & 0xffffu);
+                    } else
 #pragma unroll
                     for (int c = 0; c < CH; c += 2) {
                         asm volatile("st.shared.u16 [%0], %1;" ::"r"(qs_u + xo[c & 7] + (uint32_t)(c * 128)), "h"((unsigned short)(yr[c / 2] & 0xffffu)) : "memory");
@@ -346,33 +358,10 @@ gcg_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ C
             }
         }
     } else if (warp == W_ST) {
-        if (a.y_plain) {
-            // ======== stores of rows that no TMA box can hold: 64 bytes of a row at a time, sample by sample ==============
-            bool ok = true;
-            for (int t = 0; t < nmine && ok; ++t) {
-                const int64_t d0 = (int64_t)item_blk(t) * CH;
-                for (int k = 1; k < nchunk; ++k, ++oc) {
-                    const int qs = oc % NQ;
-                    if (!mbar_wait(y_ready(qs), (oc / NQ) & 1u, 45)) { ok = false; break; }
-#pragma unroll 1
-                    for (int s = 0; s < NS; ++s) {
-                        const Stream st = stream_of(a, item_quad(t), s);
-                        const int64_t x = st.ts + (k - 1) * CHUNK, left = st.active ? a.L - x : 0;
-                        unsigned short* const y = reinterpret_cast<unsigned short*>(a.y) + st.b * a.y_stride_b + d0 * a.y_stride_d + x;
-#pragma unroll 8
-                        for (int c = 0; c < CH; ++c)
-#pragma unroll
-                            for (int m = lane; m < CHUNK; m += 32)
-                                if (m < left) {
-                                    unsigned short v;
-                                    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(sm_u + OFF_Q + qs * TILE + tile_off(s * CH + c, m)));
-                                    y[c * a.y_stride_d + m] = v;
-                                }
-                    }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(q_empty(qs));
-                }
-            }
+        if (PLAIN) {
+            // ======== the epilogue has stored the outputs itself: a stage is free once all its warps have read it =========
+            for (oc = 0; oc < (uint32_t)(nmine * (nchunk - 1)) && mbar_wait(y_ready(oc % NQ), (oc / NQ) & 1u, 45); ++oc)
+                if (lane == 0) mbar_arrive(q_empty(oc % NQ));
         } else if (lane == 0) {
             // ======== stores: a warp of their own.  Issuing a box takes a thread ~300 cycles, two to eight of them per chunk,
             // and in an epilogue warp that held up the accumulator and the k*v slot of the whole CTA. ===================
@@ -582,36 +571,37 @@ int gcg_tc_fwd(const vtx_gcg_params* p, cudaStream_t stream) {
         if (int rc = make_tmap_bhdl(&tm[i], ptrs[i], VTX_BF16, p->L, p->head_dim, p->D / p->head_dim, p->B, sd[i], sh[i], sb[i],
                                     64, CH, a.batch_quads ? NS : 1, "gcg(tensor cores)"))
             return rc;
-    // y on 16-byte rows leaves by TMA; a dense y of an odd length (operands on padded rows) by plain stores
+    // y on 16-byte rows leaves by TMA, a dense y of an odd length (operands on padded rows) by the epilogue's own stores
+    const bool plain = reinterpret_cast<uintptr_t>(p->y) % 16 || p->y_stride_d <= 0 || p->y_stride_d % 8 ||
+                       (p->B > 1 && (p->y_stride_b <= 0 || p->y_stride_b % 8));
     CUtensorMap tmy = tm[0];
-    a.y_plain = reinterpret_cast<uintptr_t>(p->y) % 16 || p->y_stride_d <= 0 || p->y_stride_d % 8 ||
-                (p->B > 1 && (p->y_stride_b <= 0 || p->y_stride_b % 8));
-    if (!a.y_plain)
+    if (!plain)
         if (int rc = make_tmap_bhdl(&tmy, p->y, VTX_BF16, p->L, p->D, 1, p->B, p->y_stride_d, p->y_stride_d * p->D, p->y_stride_b,
                                     64, CH, a.batch_quads ? NS : 1, "gcg(tensor cores, y)"))
             return rc;
+    auto kern = plain ? gcg_tc_kernel<true> : gcg_tc_kernel<false>;
     a.hdy = p->D;
-    static bool attr_set[64] = {};
+    static bool attr_set[2][64] = {};
     static int resident[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     const bool known = dev >= 0 && dev < 64;
-    if (!known || !attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(gcg_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    if (!known || !attr_set[plain][dev]) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
         if (e != cudaSuccess) return fail(VTX_ERR_LAUNCH, "gcg(tensor cores): shared memory opt-in: %s", cudaGetErrorString(e));
-        if (known) attr_set[dev] = true;
+        if (known) attr_set[plain][dev] = true;
     }
     int nres = known ? resident[dev] : 0;
     if (nres == 0) {
         int sms = 0, per_sm = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gcg_tc_kernel, THREADS, SMEM_BYTES);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS, SMEM_BYTES);
         nres = sms * per_sm;
         if (nres <= 0) return fail(VTX_ERR_LAUNCH, "gcg(tensor cores): the kernel does not fit an SM");
         if (known) resident[dev] = nres;
     }
     const int64_t ncta = a.nitems < nres ? a.nitems : nres;
-    gcg_tc_kernel<<<(unsigned)ncta, THREADS, SMEM_BYTES, stream>>>(tm[0], tm[1], tm[2], tmy, a);
+    kern<<<(unsigned)ncta, THREADS, SMEM_BYTES, stream>>>(tm[0], tm[1], tm[2], tmy, a);
     return check_launch("gcg(tensor cores)");
 }
 

@@ -14,9 +14,10 @@
 // Time is contiguous, so a lane's samples lie in a row of their own: the warp moves tiles of 32 rows x 32 samples through
 // shared memory (16-byte asynchronous copies, one tile ahead; rows padded by 16 bytes, which makes the lanes' 16-byte
 // reads of their own rows conflict-free), and the outputs leave the same way.  Rows whose start or pitch is not a
-// multiple of 16 bytes are fetched element by element, 32 samples of a row at a time.  Bound by the issue of the fp32
-// pipe like the channel-last kernels (fused_li_cc.cu).  B=1, L=4001, D=4096, bf16: 98 us (226 us on unaligned rows); a
-// thread per row that read its own 16 bytes, 4 segments: 510 us (1130 us).
+// multiple of 16 bytes are fetched or stored element by element, 32 samples of a row at a time.  Bound by the issue of the
+// fp32 pipe like the channel-last kernels (fused_li_cc.cu).  B=1, L=4001, D=4096, bf16: 94 us from and to aligned rows, 96
+// to dense ones (117 when every store waited for its own shared-memory read), 221 from and to dense ones; a thread per row
+// that read its own 16 bytes, 4 segments: 510 us (1130 us).
 #include "common.cuh"
 #include "modal.cuh"
 
@@ -203,9 +204,18 @@ __global__ void __launch_bounds__(ITHREADS) iir_walk_kernel(vtx_iir_params p, Ii
                     }
                 }
             } else if (t + lane < t1) {
-#pragma unroll 8
-                for (int r = 0; r < 32; ++r)
-                    if (c0 + r < p.D) y[(c0 + r) * p.y_stride_d + t + lane] = *reinterpret_cast<const T*>(out + r * PITCH + lane * sizeof(T));
+                T* dst = y + c0 * p.y_stride_d + t + lane;
+                const uint8_t* from = out + lane * sizeof(T);
+                const int nrow = c0 + 32 <= p.D ? 32 : (int)(p.D - c0);
+#pragma unroll 1
+                for (int r0 = 0; r0 < nrow; r0 += 16, from += 16 * PITCH) {
+                    T e[16];
+#pragma unroll
+                    for (int r = 0; r < 16; ++r) e[r] = *reinterpret_cast<const T*>(from + r * PITCH);
+#pragma unroll
+                    for (int r = 0; r < 16; ++r, dst += p.y_stride_d)
+                        if (r0 + r < nrow) *dst = e[r];
+                }
             }
             __syncwarp();
         }
