@@ -256,6 +256,15 @@ def test_backward_tensor_core_exact_on_integers(bs, l, g, dg, hl, views):
     assert torch.equal(dh, dw.view(g, dg, hl).sum(1).flip(1))
 
 
+def same_where_not_finite(label, got, want, tol):
+    """Equal NaNs, equal infinities, and the finite rest within tol (relative L2)."""
+    got, want = got.double(), want.double()
+    assert torch.equal(got.isnan(), want.isnan()), f"{label}: NaN at {(got.isnan() != want.isnan()).nonzero()[:4].tolist()}"
+    assert torch.equal(got.isposinf(), want.isposinf()) and torch.equal(got.isneginf(), want.isneginf()), label
+    ok = want.isfinite()
+    check(label, rel_l2(got[ok], want[ok]), tol)
+
+
 @pytest.mark.parametrize("bs,l,g,dg,hl", [(1, 1, 1, 16, 4), (2, 127, 3, 16, 128), (3, 129, 2, 32, 7), (1, 1000, 20, 16, 33)])
 def test_training_forward_saves_the_filter_output(bs, l, g, dg, hl):
     """The training forward's one launch against its definition, bit for bit: y2 = xcorr(h, B * x) rounded, y = C * y2
@@ -574,6 +583,33 @@ def test_outputs_of_an_odd_length_are_dense(eng, B, L, D, K):
     ops.iir_fwd_noalloc(z, lp, res, bias, D, y, None)
     ops.iir_fwd_noalloc(z, lp, res, bias, D, again, None)
     assert torch.equal(y, again)
+
+
+@pytest.mark.parametrize("B,L,D,K", [(1, 4001, 32, 128), (2, 131, 16, 128), (3, 263, 48, 7), (5, 264, 32, 128), (1, 2000, 16, 33)])
+def test_products_that_are_not_finite_stay_under_the_filter(eng, B, L, D, K):
+    """Infinite and NaN samples in the tensor-core gate-conv-gate call: outputs they do not reach through the filter's taps
+    (earlier ones above all) are what they are without them, the others are the infinities and NaNs of the sum."""
+    g = torch.Generator(device="cuda").manual_seed(K + L)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    z = torch.zeros(B, 3 * D, (L + 7) // 8 * 8, device="cuda", dtype=torch.bfloat16)[..., :L]
+    z.copy_(r(B, 3 * D, L))
+    q, k, v = z[:, :D], z[:, D:2 * D], z[:, 2 * D:]
+    inf = float("inf")
+    k[0, 0, 0], k[0, 1, L - 1], v[0, 2, 60], v[B - 1, 3, 127], k[B - 1, 3, 128] = inf, -inf, float("nan"), inf, -inf
+    k[B - 1, 5, 40], v[B - 1, 5, 40] = 3e38, -3e38                        # finite operands, infinite product
+    k[0, 7], v[0, 7] = inf, 1                                             # a whole row
+    k[B - 1, 9], v[B - 1, 9] = float("nan"), 1
+    h = (r(D // 16, 1, K) / K ** 0.5).bfloat16()
+    bias = r(D).bfloat16()
+    y, _ = eng.parallel_fir(F.conv1d, z, h.repeat_interleave(16, 0), bias, L, dims=(D, 1, D, 16, D // 16), groups=D // 16,
+                            gated_bias=True, dim_last=False, fir_length=K, gate=True, inference_params=True)
+    kv = (k * v).double()
+    w = h[:, 0].repeat_interleave(16, 0).double()
+    w = w if K >= 128 else w.flip(1)                                       # by lag
+    acc = bias.double()[:, None] * kv
+    for j in range(min(K, L)):
+        acc[..., j:] += w[:, j, None] * kv[..., :L - j]
+    same_where_not_finite(f"gate-conv-gate with infinities L={L} K={K}", y, q.double() * acc, 8e-3)
 
 
 def test_padding_mask_and_errors(eng):

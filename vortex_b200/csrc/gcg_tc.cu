@@ -71,6 +71,8 @@ struct Args {
     int64_t hdy;                           // "head" size of the output's tensor map (D: y has one channel pitch)
     int64_t nseg, seg_len, nquad, nitems, nblk;   // nblk = D / 16 channel blocks
     int taps, bias_mode, batch_quads;      // batch_quads: mode A
+    const __nv_bfloat16 *q, *k, *v;        // the operands, for outputs that are formed without the contraction
+    int64_t q_stride_b, q_stride_h, q_stride_d, k_stride_b, k_stride_h, k_stride_d, v_stride_b, v_stride_h, v_stride_d;
 };
 
 struct Stream {
@@ -103,6 +105,47 @@ __device__ __forceinline__ uint32_t instr_desc_kmajor(int M, int N) {
 // byte offset of (column n, sample t) in a tile
 __device__ __forceinline__ uint32_t tile_off(int n, int t) {
     return (uint32_t)((t >> 6) * HALF_TILE + n * 128 + ((((t & 63) >> 3) ^ (n & 7)) << 4) + (t & 7) * 2);
+}
+
+// Outputs whose filter sums are not all finite, again and under the filter's taps only: the contraction multiplies every
+// product of its 256-sample window, and a zero tap times infinity or NaN is NaN.  Sample r of the chunk of quad that starts
+// dt samples into its segments, in 16 channels of streams s0 and s0 + 1; taps and skip parameters as the epilogue has them.
+// The results go to y (PLAIN) or over the q tile.
+template <bool PLAIN>
+__device__ __noinline__ void outputs_under_taps(const Args& a, const uint16_t* taps, const float* dsk, uint32_t tile, int blk, int64_t quad,
+                                                int64_t dt, int r, int s0) {
+    using bf = __nv_bfloat16;
+    const int K = (int)a.K;
+#pragma unroll 1
+    for (int s = s0; s < s0 + 2; ++s) {
+        const Stream st = stream_of(a, quad, s);
+        const int64_t t = st.ts + dt + r;
+        if (!st.active) continue;
+#pragma unroll 1
+        for (int c = 0; c < CH; ++c) {
+            const int64_t d = (int64_t)blk * CH + c, head = d / a.hd, row = d % a.hd;
+            const bf* const kr = a.k + st.b * a.k_stride_b + head * a.k_stride_h + row * a.k_stride_d;
+            const bf* const vr = a.v + st.b * a.v_stride_b + head * a.v_stride_h + row * a.v_stride_d;
+            const bool in = t < a.L;
+            float sum = 0.f;
+            for (int j0 = 0; j0 < K; j0 += 8) {
+#pragma unroll
+                for (int j = j0; j < j0 + 8; ++j)
+                    if (in && j < K && j <= t)
+                        sum = fmaf(__uint_as_float((uint32_t)taps[j] << 16), round_io<bf>(__bfloat162float(kr[t - j]) * __bfloat162float(vr[t - j])), sum);
+                if (__all_sync(0xffffffffu, isnan(sum) || !in)) break;
+            }
+            if (!in) continue;
+            if (a.bias_mode == VTX_BIAS_GATED) {
+                const float kv = round_io<bf>(__bfloat162float(kr[t]) * __bfloat162float(vr[t]));
+                sum = a.taps == VTX_TAPS_CONV ? fmaf(dsk[c], kv, sum) : round_io<bf>(sum) + round_io<bf>(dsk[c] * kv);
+            }
+            const float q = __bfloat162float(a.q[st.b * a.q_stride_b + head * a.q_stride_h + row * a.q_stride_d + t]);
+            const bf y = __float2bfloat16_rn(q * round_io<bf>(sum));
+            if (PLAIN) a.y[st.b * a.y_stride_b + d * a.y_stride_d + t] = y;
+            else asm volatile("st.shared.u16 [%0], %1;" ::"r"(tile + tile_off(s * CH + c, r)), "h"(__bfloat16_as_ushort(y)) : "memory");
+        }
+    }
 }
 
 // PLAIN: y's rows do not start on 16-byte boundaries, so no tensor map holds them
@@ -289,6 +332,8 @@ gcg_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ C
                 // every pair paid the round trip of its loads (3600 of 4250 cycles per chunk, which everything else then
                 // waited for).
                 const bool skip = a.bias_mode == VTX_BIAS_GATED;
+                f32x2 finite = 0;              // sums times zero: zero, or NaN once one of them is not finite (217 -> 221 us at
+                                               // B=4, L=8192; a check of every stream before its gate: 232)
 #pragma unroll 1
                 for (int s = 2 * sh; s < 2 * sh + 2; ++s) {
                     uint32_t acc[16], qv[16], kvv[16];
@@ -325,6 +370,7 @@ gcg_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ C
                                 z = add2(pk2(bf_lo(zr), bf_hi(zr)), pk2(bf_lo(br), bf_hi(br)));
                             }
                         }
+                        finite = fma2(z, 0, finite);
                         float z0, z1;
                         up2(z, z0, z1);
                         const uint32_t zr = pack_bf16(z0, z1);                 // the filter output in the I/O dtype
@@ -350,6 +396,11 @@ gcg_tc_kernel(const __grid_constant__ CUtensorMap tmq, const __grid_constant__ C
                         asm volatile("st.shared.u16 [%0], %1;" ::"r"(qs_u + xo[(c + 1) & 7] + (uint32_t)((c + 1) * 128)), "h"((unsigned short)(yr[c / 2] >> 16)) : "memory");
                     }
                 }
+                float f0, f1;
+                up2(finite, f0, f1);
+                if (__any_sync(0xffffffffu, f0 + f1 != 0.f))
+                    outputs_under_taps<PLAIN>(a, reinterpret_cast<const uint16_t*>(smp(OFF_TAPS + (t & 1) * 768)) + 128, dsk, sm_u + OFF_Q + qs * TILE,
+                                              blk, item_quad(t), (int64_t)(k - 1) * CHUNK, r, 2 * sh);
                 // k*v has been read: the slot may go; the tile of outputs goes to the TMA unit once all four warps wrote it
                 fence_proxy_async_smem();
                 __syncwarp();
@@ -543,6 +594,11 @@ int gcg_tc_fwd(const vtx_gcg_params* p, cudaStream_t stream) {
     a.state = (p->state && p->K > 1) ? static_cast<__nv_bfloat16*>(p->state) : nullptr;
     a.B = p->B; a.L = p->L; a.D = p->D; a.K = p->K; a.dg = p->D / p->G; a.hd = p->head_dim;
     a.taps = (int)p->taps; a.bias_mode = (int)p->bias_mode;
+    a.q = static_cast<const __nv_bfloat16*>(p->q); a.k = static_cast<const __nv_bfloat16*>(p->k);
+    a.v = static_cast<const __nv_bfloat16*>(p->v);
+    a.q_stride_b = p->q_stride_b; a.q_stride_h = p->q_stride_h; a.q_stride_d = p->q_stride_d;
+    a.k_stride_b = p->k_stride_b; a.k_stride_h = p->k_stride_h; a.k_stride_d = p->k_stride_d;
+    a.v_stride_b = p->v_stride_b; a.v_stride_h = p->v_stride_h; a.v_stride_d = p->v_stride_d;
     a.nblk = p->D / CH;
     a.batch_quads = p->B >= 3;
     // time segments: as in the fused kernel, the launch lasts as long as the CTA with the most chunks
