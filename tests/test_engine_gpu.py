@@ -265,6 +265,44 @@ def same_where_not_finite(label, got, want, tol):
     check(label, rel_l2(got[ok], want[ok]), tol)
 
 
+@pytest.mark.parametrize("bs,l,g,dg,hl,big", [
+    (1, 130, 1, 16, 128, False), (2, 700, 3, 16, 128, False), (1, 2100, 2, 32, 7, False), (3, 300, 1, 48, 33, False),
+    (1, 300, 160, 16, 128, False), (2, 200, 1, 16, 128, True)])
+def test_backward_products_that_are_not_finite_stay_under_the_filter(bs, l, g, dg, hl, big):
+    """Infinite and NaN operands of the tensor-core backward: the gradients they do not reach through the filter's taps are
+    what they are without them, the others are the infinities and NaNs of the sums.  ``big``: finite products that round to
+    an infinite bf16 head stay finite."""
+    from vortex_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(hl + l)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=gen).bfloat16()  # noqa: E731
+    D, inf = g * dg, float("inf")
+    dy, x, Bm, Cm, y2 = (r(bs, l, D) for _ in range(5))
+    h = (0.1 * r(g, hl).float() / hl ** 0.5).bfloat16()
+    if big:                        # 181 / 128 squared is 2 - 2^-8.5: below the fp32 maximum, above the bf16 one
+        x, Bm = x * 1e-3, Bm * 1e-3
+        dy[0, 40, 3], Cm[0, 40, 3] = 181 / 128 * 2. ** 63, 181 / 128 * 2. ** 64
+        dy[-1, l - 1, 7], Cm[-1, l - 1, 7] = -181 / 128 * 2. ** 64, 181 / 128 * 2. ** 63
+    else:
+        dy[0, 0, 0], Cm[0, l - 1, 1], dy[-1, 127, 2], dy[-1, 128, 2], Cm[0, 60, 3] = inf, -inf, inf, -inf, float("nan")
+        x[-1, 64, D - 1], Bm[-1, l // 2, D - 2], x[0, l - 1, D - 3] = inf, float("nan"), -inf
+        dy[0, :, 5] = inf
+    dx, dB, dC, dh = ops.gcg_bwd(dy, x, Bm, Cm, y2, h)
+    g2, z, w = (dy.float() * Cm.float()).double(), (x.float() * Bm.float()).double(), h.double().flip(1).repeat_interleave(dg, 0)
+    dz, dw = torch.zeros_like(g2), torch.zeros(D, hl, dtype=torch.double, device="cuda")
+    for j in range(min(hl, l)):
+        dz[:, :l - j] += w[:, j] * g2[:, j:]
+        dw[:, j] = (g2[:, j:] * z[:, :l - j]).sum((0, 1))
+    for name, got, want, tol in (("dx", dx, dz * Bm.double(), 4e-3), ("dB", dB, dz * x.double(), 4e-3),
+                                 ("dC", dC, dy.double() * y2.double(), 4e-3), ("dh", dh, dw.view(g, dg, hl).sum(1).flip(1), 1e-5)):
+        if big:                    # the huge values (and the sums that hold them) apart from the rest
+            huge = want.abs() > 1e25
+            assert huge.any() or name == "dC"
+            same_where_not_finite(f"{name} huge", got[huge].double() * 1e-30, want[huge] * 1e-30, tol)
+            got, want = got[~huge], want[~huge]
+        same_where_not_finite(f"backward with infinities {name} l={l} hl={hl}", got, want, tol)
+
+
 @pytest.mark.parametrize("bs,l,g,dg,hl", [(1, 1, 1, 16, 4), (2, 127, 3, 16, 128), (3, 129, 2, 32, 7), (1, 1000, 20, 16, 33)])
 def test_training_forward_saves_the_filter_output(bs, l, g, dg, hl):
     """The training forward's one launch against its definition, bit for bit: y2 = xcorr(h, B * x) rounded, y = C * y2

@@ -15,8 +15,9 @@
 // Precision.  g2 and z are products of two bf16 numbers: 16 significant bits, so head + remainder in bf16 hold them EXACTLY
 // (the fp32 kernels of gcg_bwd.cu work on the same exact products).  Taps are bf16, accumulation is fp32, one rounding on
 // the way out.  dw takes all four products of heads and remainders.
-// An infinite or NaN product makes its channel's dz NaN over the 256 rows of the contraction's window, not only under the
-// filter's taps (a zero tap times infinity), as in the forward kernel.
+// A product that is infinite or NaN (or whose head rounds to infinity: a finite one above the bf16 maximum of 3.39e38) would
+// make dz NaN over the 256 rows of the contraction's window and dh at every lag; the sums it reaches are formed again under
+// the taps alone (dz_under_taps, dw_under_taps).  Products below 2^-117 have remainders below bf16's subnormals, which are lost.
 //
 // What bounds it: 10 bytes in and 6 bytes out per element (B=2, L=8192, D=4096: 1.07 GB = 164 us at 6.54 TB/s), i.e. 2900
 // cycles per chunk and SM, of which the tensor pipe needs 16 x 85 (dz) + 8 x 128 (dw) and shared memory about as many.
@@ -64,6 +65,9 @@ struct Args {
     int64_t B, L, D, G, K;       // G: groups of 16 channels
     int64_t dg;                  // channels that share a filter (a multiple of 16)
     int64_t nseg, seg_len, nstream, nset, nitems, item0, item1;
+    // the operands, for the sums that are not contracted
+    const __nv_bfloat16 *dy, *x, *Bg, *C;
+    int64_t dy_sb, dy_sl, x_sb, x_sl, b_sb, b_sl, c_sb, c_sl;
 };
 
 struct Stream { int b, ts, te; bool active; };
@@ -103,6 +107,54 @@ __device__ __forceinline__ void split_tile(uint32_t tile, int r, int c, const ui
 __device__ __forceinline__ uint32_t mul_pair(uint32_t a, uint32_t b) { return pack_bf16(bf_lo(a) * bf_lo(b), bf_hi(a) * bf_hi(b)); }
 
 struct Maps { CUtensorMap dy, x, Bg, C, y2; };
+
+// The sums under the filter's taps alone, in fp32 on the exact products: the contractions multiply every row of their
+// windows, and a zero times infinity or NaN is NaN.  A warp whose sums are not all finite takes these instead.  (Among them
+// finite products whose head rounds to infinity.)
+__device__ __forceinline__ void mul_rows(const __nv_bfloat16* p, const __nv_bfloat16* q, float (&out)[CH]) {
+    const uint4 a0 = reinterpret_cast<const uint4*>(p)[0], a1 = reinterpret_cast<const uint4*>(p)[1];
+    const uint4 b0 = reinterpret_cast<const uint4*>(q)[0], b1 = reinterpret_cast<const uint4*>(q)[1];
+    const uint32_t aw[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, bw[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { out[2 * j] = bf_lo(aw[j]) * bf_lo(bw[j]); out[2 * j + 1] = bf_hi(aw[j]) * bf_hi(bw[j]); }
+}
+// dz at row t of 16 channels from c0 on (rows past the end are not stored)
+__device__ __noinline__ void dz_under_taps(const Args& a, int64_t b, int64_t c0, int64_t t, uint32_t* out) {
+    const __nv_bfloat16* const w = a.h + (c0 / a.dg) * a.K + a.K - 1;
+    float sum[CH] = {};
+    for (int64_t j = 0; j < a.K; ++j) {
+        bool done = true;
+        if (t + j < a.L) {
+            float g2[CH];
+            mul_rows(a.dy + b * a.dy_sb + (t + j) * a.dy_sl + c0, a.C + b * a.c_sb + (t + j) * a.c_sl + c0, g2);
+            const float wj = __bfloat162float(w[-j]);
+#pragma unroll
+            for (int c = 0; c < CH; ++c) { sum[c] = fmaf(wj, g2[c], sum[c]); done = done && isnan(sum[c]); }
+        }
+        if (__all_sync(0xffffffffu, done)) break;
+    }
+#pragma unroll
+    for (int c = 0; c < CH; ++c) out[c] = __float_as_uint(sum[c]);
+}
+// sum over rows ts .. te - 1 that are rows first .. first + 31 of their chunk, and 16 channels, of g2[t] z[t - lag]
+__device__ __noinline__ float dw_under_taps(const Args& a, int64_t b, int64_t c0, int ts, int te, int first, int lag) {
+    float total = 0.f;
+    for (int t0 = ts + first; t0 < te; t0 += CHUNK) {
+        float sum = 0.f;
+#pragma unroll 4
+        for (int t = t0; t < t0 + 32; ++t) {
+            if (t >= te || t < lag || lag >= a.K) continue;
+            float g2[CH], z[CH];
+            mul_rows(a.dy + b * a.dy_sb + t * a.dy_sl + c0, a.C + b * a.c_sb + t * a.c_sl + c0, g2);
+            mul_rows(a.x + b * a.x_sb + (t - lag) * a.x_sl + c0, a.Bg + b * a.b_sb + (t - lag) * a.b_sl + c0, z);
+#pragma unroll
+            for (int c = 0; c < CH; ++c) sum = fmaf(g2[c], z[c], sum);
+        }
+        total += sum;
+        if (__all_sync(0xffffffffu, isnan(total) || lag >= a.K)) break;
+    }
+    return total;
+}
 
 __global__ void __launch_bounds__(THREADS, 1) gcg_bwd_tc_kernel(const __grid_constant__ Maps maps, const __grid_constant__ Args a) {
     extern __shared__ uint8_t smem_raw[];
@@ -276,6 +328,25 @@ __global__ void __launch_bounds__(THREADS, 1) gcg_bwd_tc_kernel(const __grid_con
                     }
                     const int64_t yo = (s ? yoff[1] : yoff[0]) + step;
                     const int nl = s ? nleft[1] : nleft[0];
+                    // (sums times zero are zero, or NaN if one of them is not finite)
+                    f32x2 dz[CH / 2], finite = 0;
+#pragma unroll
+                    for (int j = 0; j < CH / 2; ++j) {
+                        dz[j] = add2(pk2(__uint_as_float(ah[2 * j]), __uint_as_float(ah[2 * j + 1])),
+                                     pk2(__uint_as_float(al[2 * j]), __uint_as_float(al[2 * j + 1])));
+                        finite = fma2(dz[j], 0, finite);
+                    }
+                    float f0, f1;
+                    up2(finite, f0, f1);
+                    if (__any_sync(0xffffffffu, f0 + f1 != 0.f)) {
+                        const Stream st = stream_of(a, item_set(t), s);
+                        uint32_t sums[CH];
+                        if (st.active) {
+                            dz_under_taps(a, st.b, (int64_t)g * CH, st.ts + (int64_t)(k - 1) * CHUNK + tt, sums);
+#pragma unroll
+                            for (int j = 0; j < CH / 2; ++j) dz[j] = pk2(__uint_as_float(sums[2 * j]), __uint_as_float(sums[2 * j + 1]));
+                        }
+                    }
                     uint32_t ox[8], ob[8];
 #pragma unroll
                     for (int hf = 0; hf < 2; ++hf) {
@@ -283,8 +354,8 @@ __global__ void __launch_bounds__(THREADS, 1) gcg_bwd_tc_kernel(const __grid_con
                         const uint32_t xw[4] = {x4.x, x4.y, x4.z, x4.w}, bw[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
-                            const float d0 = __uint_as_float(ah[8 * hf + 2 * j]) + __uint_as_float(al[8 * hf + 2 * j]);
-                            const float d1 = __uint_as_float(ah[8 * hf + 2 * j + 1]) + __uint_as_float(al[8 * hf + 2 * j + 1]);
+                            float d0, d1;
+                            up2(dz[4 * hf + j], d0, d1);
                             ox[4 * hf + j] = pack_bf16(d0 * bf_lo(bw[j]), d1 * bf_hi(bw[j]));
                             ob[4 * hf + j] = pack_bf16(d0 * bf_lo(xw[j]), d1 * bf_hi(xw[j]));
                         }
@@ -335,13 +406,21 @@ __global__ void __launch_bounds__(THREADS, 1) gcg_bwd_tc_kernel(const __grid_con
                 tc_fence_before();
                 __syncwarp();
                 float* const dh = a.dh + (int64_t)((unsigned)(g * CH) / (unsigned)a.dg) * K;
-#pragma unroll
+#pragma unroll 1
                 for (int lag = lane; lag < CHUNK; lag += 32) {
                     float v = 0.f;
 #pragma unroll
                     for (int q = 0; q < RUNS; ++q) {
                         const int m = lag - RUN * q + 31;
                         if (m >= 0 && m < RUN_LAGS) v += sums[q * RUN_LAGS + m];
+                    }
+                    if (__any_sync(0xffffffffu, lag < K && !isfinite(v))) {
+                        v = 0.f;
+#pragma unroll 1
+                        for (int s = 0; s < NS; ++s) {
+                            const Stream st = stream_of(a, item_set(t), s);
+                            if (st.active) v += dw_under_taps(a, st.b, (int64_t)g * CH, st.ts, st.te, CHUNK - 32 * (e + 1), lag);
+                        }
                     }
                     if (lag < K) atomicAdd(dh + (K - 1 - lag), v);
                 }
@@ -505,6 +584,10 @@ int launch(const vtx_gcg_bwd_params* p, cudaStream_t stream) {
     a.h = static_cast<const __nv_bfloat16*>(p->h);
     a.dx = static_cast<__nv_bfloat16*>(p->dx); a.dB = static_cast<__nv_bfloat16*>(p->dB); a.dC = static_cast<__nv_bfloat16*>(p->dC);
     a.dh = p->dh32;
+    a.dy = static_cast<const __nv_bfloat16*>(p->dy); a.x = static_cast<const __nv_bfloat16*>(p->x);
+    a.Bg = static_cast<const __nv_bfloat16*>(p->Bg); a.C = static_cast<const __nv_bfloat16*>(p->C);
+    a.dy_sb = p->dy_stride_b; a.dy_sl = p->dy_stride_l; a.x_sb = p->x_stride_b; a.x_sl = p->x_stride_l;
+    a.b_sb = p->b_stride_b; a.b_sl = p->b_stride_l; a.c_sb = p->c_stride_b; a.c_sl = p->c_stride_l;
     a.B = p->B; a.L = p->L; a.D = p->D; a.G = p->D / CH; a.K = p->K; a.dg = p->D / p->G;
     plan_items(a);
     Maps maps;
