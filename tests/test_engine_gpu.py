@@ -303,6 +303,53 @@ def test_backward_products_that_are_not_finite_stay_under_the_filter(bs, l, g, d
         same_where_not_finite(f"backward with infinities {name} l={l} hl={hl}", got, want, tol)
 
 
+@pytest.mark.parametrize("l,d,hl", [(8192, 512, 128), (131072, 512, 32), (1024, 768, 7)])
+def test_backward_filter_gradient_on_long_sequences(l, d, hl):
+    """dh against 64 bits.  Bound: the tensor core truncates an accumulator 16 times (two chunks of eight steps, ten of
+    them onto a sum that is not small) by half of 2^-23 on average, 6e-8 each with random signs: 2e-7, doubled; fp32 sums
+    in the CUDA cores' kernels measure 3e-7 to 5e-7, a sum over whole items 1e-6 to 9e-6."""
+    from vortex_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(l)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=gen).bfloat16()  # noqa: E731
+    dy, x, Bm, Cm, y2 = (r(1, l, d) for _ in range(5))
+    dh = ops.gcg_bwd(dy, x, Bm, Cm, y2, r(d // 16, hl))[3]
+    g2, z = dy.double() * Cm.double(), x.double() * Bm.double()
+    ref = torch.stack([(g2[:, j:] * z[:, :l - j]).sum((0, 1)).view(-1, 16).sum(1) for j in range(hl)], 1).flip(1)
+    check(f"dh of a long sequence l={l} hl={hl}", float((dh.double() - ref).norm() / ref.norm()), 4e-7)
+
+
+@pytest.mark.parametrize("bs,l,g,hl", [(2, 4100, 256, 128), (1, 5000, 20, 33), (400, 128, 256, 128)])
+def test_backward_tensor_core_exact_on_long_walks(bs, l, g, hl):
+    """Items of many chunks, several items per CTA, and a call cut into two launches (51200 items of one chunk): small
+    integers, all four gradients exact (see test_backward_tensor_core_exact_on_integers)."""
+    from vortex_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    D = g * 16
+    ri = lambda lo, hi, *sh: torch.randint(lo, hi + 1, sh, device="cuda", generator=gen).to(torch.bfloat16)  # noqa: E731
+    dy, x, Bm, Cm = ri(-2, 2, bs, l, D), ri(-1, 1, bs, l, D), ri(-1, 1, bs, l, D), ri(-1, 1, bs, l, D)
+    h = ri(-1, 1, g, hl)
+    if hl > 64:
+        h[:, 32:hl - 32] = 0
+    before = ops.launch_count()
+    dx, dB, dC, dh = ops.gcg_bwd(dy, x, Bm, Cm, x, h)
+    assert ops.launch_count() - before == (2 if bs == 400 else 1)
+    w = h.flip(1).repeat_interleave(16, 0).double()
+    dw = torch.zeros(D, hl, dtype=torch.double, device="cuda")
+    for b in range(0, bs, 40):                                      # (64-bit tensors of a part of the batch at a time)
+        p = slice(b, b + 40)
+        g2, z = dy[p].double() * Cm[p].double(), x[p].double() * Bm[p].double()
+        dz = torch.zeros_like(g2)
+        for j in range(min(hl, l)):
+            dz[:, :l - j] += w[:, j] * g2[:, j:]
+            dw[:, j] += (g2[:, j:] * z[:, :l - j]).sum((0, 1))
+        assert dz.abs().max() <= 256
+        assert torch.equal(dx[p].double(), dz * Bm[p].double()) and torch.equal(dB[p].double(), dz * x[p].double())
+        assert torch.equal(dC[p].double(), dy[p].double() * x[p].double())
+    assert torch.equal(dh.double(), dw.view(g, 16, hl).sum(1).flip(1))
+
+
 @pytest.mark.parametrize("bs,l,g,dg,hl", [(1, 1, 1, 16, 4), (2, 127, 3, 16, 128), (3, 129, 2, 32, 7), (1, 1000, 20, 16, 33)])
 def test_training_forward_saves_the_filter_output(bs, l, g, dg, hl):
     """The training forward's one launch against its definition, bit for bit: y2 = xcorr(h, B * x) rounded, y = C * y2

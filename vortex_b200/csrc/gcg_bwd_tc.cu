@@ -9,26 +9,27 @@
 //   dz    blocked Toeplitz: the chunk's g2 is stored with time REVERSED, which turns the anti-causal filter into the causal
 //         operand [T^ | T][i][j] = w[128 + i - j] of the forward kernel, here applied to (next chunk, this chunk).
 //   dw    W[i][i'] += sum over the 32 columns of g2[i] z[i'] for the chunk's 128 rows of g2 against the 256 rows of z that
-//         end with the chunk: an ordinary M128 x N256 contraction of K-major tiles, accumulated in TMEM over ALL chunks of
-//         the item; dw[j] is the sum along an anti-diagonal of W, taken once per item.
+//         end with the chunk: an ordinary M128 x N256 contraction of K-major tiles, accumulated in TMEM over two chunks;
+//         dw[j] is the sum along an anti-diagonal of W, kept in fp32 registers over the item.
 //
-// Precision.  g2 and z are products of two bf16 numbers: 16 significant bits, so head + remainder in bf16 hold them EXACTLY
-// (the fp32 kernels of gcg_bwd.cu work on the same exact products).  Taps are bf16, accumulation is fp32, one rounding on
+// Precision.  g2 and z are products of two bf16 numbers: 16 significant bits, so head + remainder in bf16 hold them exactly
+// between 2^-117 and 3.39e38 (the fp32 kernels of gcg_bwd.cu work on the same products; below, the remainder is cut to
+// bf16's subnormals, above, the head is infinite).  Taps are bf16, accumulation is fp32, one rounding on
 // the way out.  dw takes all four products of heads and remainders.
-// A product that is infinite or NaN (or whose head rounds to infinity: a finite one above the bf16 maximum of 3.39e38) would
-// make dz NaN over the 256 rows of the contraction's window and dh at every lag; the sums it reaches are formed again under
-// the taps alone (dz_under_taps, dw_under_taps).  Products below 2^-117 have remainders below bf16's subnormals, which are lost.
+// A product that is infinite or NaN, or whose head is, would make dz NaN over the 256 rows of the contraction's window and dh
+// at every lag; the sums it reaches are formed again under the taps alone (dz_under_taps, dw_under_taps).
 //
 // What bounds it: 10 bytes in and 6 bytes out per element (B=2, L=8192, D=4096: 1.07 GB = 164 us at 6.54 TB/s), i.e. 2900
 // cycles per chunk and SM, of which the tensor pipe needs 16 x 85 (dz) + 8 x 128 (dw) and shared memory about as many.
-// Measured: 277 us with the launch that clears the fp32 accumulator, the fp32 kernels 1290 us; B=4: 495 us = 4.3 TB/s.
+// Measured: 326 us with the launch that clears the fp32 accumulator, the fp32 kernels 1290 us; B=4: 617 us = 3.5 TB/s.  A
+// W that gathers all chunks of an item is 50 us faster and too inexact (WCHUNKS).
 // Everything arrives by TMA: with 224 KB of the SM carved out as shared memory L1 holds some 220 lines, so plain loads of
 // 32-byte row pieces kept 7 KB in flight (first version: 18000 cycles per chunk, 700 us).
 //
 // One persistent CTA per SM walks the items (strided by the launch width: concurrent CTAs read neighbouring groups of the
-// same rows).  14 warps: 0-7 front end (staged rows -> products -> tiles; dC leaves from here), 8-11 epilogue (dz out of
-// TMEM, gates, stores; at the end of an item the anti-diagonals of W, then the next item's Toeplitz operand), 12 MMA
-// issue, 13 TMA issue.  x and B stay in their stage until the epilogue, one to two chunks later, has used them.  TMEM:
+// same rows).  18 warps: 0-7 front end (staged rows -> products -> tiles; dC leaves from here), 8-11 epilogue (dz out of
+// TMEM, gates, stores; the next item's Toeplitz operand), 12 MMA issue, 13 TMA issue, 14-17 the sums along W (as a part of
+// the epilogue they cost 8 us more).  x and B stay in their stage until the epilogue, one to two chunks later, has used them.  TMEM:
 // operand 128 columns, dz 2 x 64, W 256 -- all 512.  All waits are bounded.
 #include "tma.cuh"
 #include "umma.cuh"
@@ -42,7 +43,7 @@ namespace gbt {
 using namespace umma;
 
 constexpr int NS = 2, CH = 16, CHUNK = 128;
-constexpr int NFE = 8, W_EP = NFE, W_MMA = NFE + 4, W_TMA = NFE + 5, THREADS = 32 * 14;
+constexpr int NFE = 8, W_EP = NFE, W_MMA = NFE + 4, W_TMA = NFE + 5, W_DW = NFE + 6, THREADS = 32 * 18;
 constexpr int WROWS = CHUNK / NFE;                 // rows of a chunk per front-end warp
 constexpr int TILE = CHUNK * 128;                  // [128 rows][64 columns] bf16, 128-byte swizzle
 constexpr int BOX = CHUNK * CH * 2;                // staged box: 128 rows x 16 channels of one stream and tensor
@@ -50,10 +51,16 @@ constexpr int NG = 2, NZ = 3;                      // tile rings: g2 is consumed
 constexpr int NXS = 4, NDS = 3;                    // stages of (x, B), held until the epilogue is done, and of (dy, C, y2)
 constexpr int X_STAGE = 2 * NS * BOX, D_STAGE = 3 * NS * BOX;
 constexpr int OFF_Z = 0, OFF_G = OFF_Z + NZ * TILE, OFF_X = OFF_G + NG * TILE, OFF_D = OFF_X + NXS * X_STAGE;
-constexpr int RUNS = 4, RUN = 40;                  // sums along the anti-diagonals of W: runs per warp, columns per run
-constexpr int RUN_LAGS = RUN + 31;                 // lags a run contributes to
+// Chunks whose products meet in W before it is read out.  The tensor core truncates an accumulator at every step, so the
+// error grows with them: dh of random operands against 64 bits, B=2, L=8192, D=4096, K=128 (L=131072, D=512): 1.6e-7
+// (2.2e-7) with one, 2.8e-7 (3.0e-7) with two, 5.6e-7 with four, 2.3e-6 (8.4e-6) over whole items; the fp32 kernels 3.3e-7
+// (5.0e-7).  Operands of one sign, whose truncations do not cancel: 8.8e-8 (1.1e-7), 2.2e-7 (2.3e-7), 5.4e-7 (5.3e-7),
+// 2.6e-6 (1.1e-5); the fp32 kernels 1.2e-7 (3.3e-7).  Time: 400, 326, 304 and 288 us.
+constexpr int WCHUNKS = 2;
+constexpr int RUNS = 4, RUN = 40;                  // sums along the anti-diagonals of W: runs per warp, most columns per run
+constexpr int RUN_LAGS = RUN + 32;                 // words of a run's sums
 constexpr int OFF_TAPS = OFF_D + NDS * D_STAGE, OFF_RUNS = OFF_TAPS + 384 * 2, OFF_BARS = OFF_RUNS + 4 * RUNS * RUN_LAGS * 4;
-constexpr int NBARS = 2 * (NG + NZ + NXS + NDS) + 4 + 3;
+constexpr int NBARS = 2 * (NG + NZ + NXS + NDS) + 4 + 4;
 constexpr int SMEM_BYTES = OFF_BARS + NBARS * 8 + 16 + 1024;
 static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
 constexpr int A_COL = 0, DZ_COL = 128, W_COL = 256, TMEM_COLS = 512;
@@ -164,7 +171,7 @@ __global__ void __launch_bounds__(THREADS, 1) gcg_bwd_tc_kernel(const __grid_con
     auto bar = [&](uint32_t first, uint32_t i) { return bar_u + 8u * (first + i); };
     constexpr uint32_t G_FULL = 0, G_FREE = G_FULL + NG, Z_FULL = G_FREE + NG, Z_FREE = Z_FULL + NZ, X_FULL = Z_FREE + NZ,
                        X_FREE = X_FULL + NXS, D_FULL = X_FREE + NXS, D_FREE = D_FULL + NDS, DZ_FULL = D_FREE + NDS, DZ_EMPTY = DZ_FULL + 2,
-                       W_FULL = DZ_EMPTY + 2, A_READY = W_FULL + 1, TAPS_READY = A_READY + 1;
+                       W_FULL = DZ_EMPTY + 2, W_EMPTY = W_FULL + 1, A_READY = W_EMPTY + 1, TAPS_READY = A_READY + 1;
     static_assert(TAPS_READY + 1 == NBARS, "barrier count");
     const uint32_t tslot = bar_u + 8u * NBARS;
 
@@ -182,7 +189,7 @@ __global__ void __launch_bounds__(THREADS, 1) gcg_bwd_tc_kernel(const __grid_con
         for (int i = 0; i < NXS; ++i) { mbar_init(bar(X_FULL, i), 1); mbar_init(bar(X_FREE, i), NFE + 4); }
         for (int i = 0; i < NDS; ++i) { mbar_init(bar(D_FULL, i), 1); mbar_init(bar(D_FREE, i), NFE); }
         for (int i = 0; i < 2; ++i) { mbar_init(bar(DZ_FULL, i), 1); mbar_init(bar(DZ_EMPTY, i), 4); }
-        mbar_init(bar(W_FULL, 0), 1); mbar_init(bar(A_READY, 0), 4); mbar_init(bar(TAPS_READY, 0), 4);
+        mbar_init(bar(W_FULL, 0), 1); mbar_init(bar(W_EMPTY, 0), 4); mbar_init(bar(A_READY, 0), 4); mbar_init(bar(TAPS_READY, 0), 4);
         fence_mbar_init();
     }
     if (warp == W_MMA) {
@@ -370,63 +377,7 @@ __global__ void __launch_bounds__(THREADS, 1) gcg_bwd_tc_kernel(const __grid_con
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar(X_FREE, xs));
             }
-            if (!ok || !mbar_wait(bar(W_FULL, 0), (uint32_t)(t & 1), 8)) { ok = false; break; }
-            tc_fence_after();
-            __syncwarp();
-            // Anti-diagonals of W: row i (g2 at time 127 - i of the chunk) and column c (z at time c - 128 of it) meet at lag
-            // 255 - i - c, so a sum that moves one lane up per column to the left stays on its lag.  Columns 96 - 32 e ..
-            // 255 - 32 e hold every lag 0..127 of this warp's rows; four independent runs of 40 columns hide the shuffle's
-            // latency.  Run q's lag 40 q - 31 + m leaves lane 31 at its column m, the last 31 lags sit in the lanes below
-            // at its end: all go to shared memory, and one sum over the runs is added to the group's dh.  (Adding each value
-            // to dh where it left lane 31 took 13 K cycles per item, most of the gap between two items.)
-            {
-                float* const sums = reinterpret_cast<float*>(smp(OFF_RUNS)) + e * RUNS * RUN_LAGS;
-                float run[RUNS] = {0.f, 0.f, 0.f, 0.f};
-                const int top = 255 - 32 * e;                      // first column of run 0; run q starts 40 q further left
-#pragma unroll 1
-                for (int c0 = 0; c0 < RUN; c0 += 8) {
-                    uint32_t w8[RUNS][8];
-#pragma unroll
-                    for (int q = 0; q < RUNS; ++q) tmem_ld8(lane_base + W_COL + (uint32_t)(top - RUN * q - c0 - 7), w8[q]);
-                    tmem_ld8_wait(w8[0], w8[1]);
-                    tmem_ld8_wait(w8[2], w8[3]);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-#pragma unroll
-                        for (int q = 0; q < RUNS; ++q) {
-                            const float up = __shfl_up_sync(0xffffffffu, run[q], 1);
-                            run[q] = (lane ? up : 0.f) + __uint_as_float(w8[q][7 - j]);
-                            if (lane == 31) sums[q * RUN_LAGS + c0 + j] = run[q];
-                        }
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < RUNS; ++q)
-                    if (lane < 31) sums[q * RUN_LAGS + RUN_LAGS - 1 - lane] = run[q];
-                tc_fence_before();
-                __syncwarp();
-                float* const dh = a.dh + (int64_t)((unsigned)(g * CH) / (unsigned)a.dg) * K;
-#pragma unroll 1
-                for (int lag = lane; lag < CHUNK; lag += 32) {
-                    float v = 0.f;
-#pragma unroll
-                    for (int q = 0; q < RUNS; ++q) {
-                        const int m = lag - RUN * q + 31;
-                        if (m >= 0 && m < RUN_LAGS) v += sums[q * RUN_LAGS + m];
-                    }
-                    if (__any_sync(0xffffffffu, lag < K && !isfinite(v))) {
-                        v = 0.f;
-#pragma unroll 1
-                        for (int s = 0; s < NS; ++s) {
-                            const Stream st = stream_of(a, item_set(t), s);
-                            if (st.active) v += dw_under_taps(a, st.b, (int64_t)g * CH, st.ts, st.te, CHUNK - 32 * (e + 1), lag);
-                        }
-                    }
-                    if (lag < K) atomicAdd(dh + (K - 1 - lag), v);
-                }
-                __syncwarp();
-            }
-            if (t + 1 < nmine && !expand(t + 1)) ok = false;
+            if (ok && t + 1 < nmine && !expand(t + 1)) ok = false;
         }
     } else if (warp == W_MMA) {
         if (lane == 0) {
@@ -443,16 +394,16 @@ __global__ void __launch_bounds__(THREADS, 1) gcg_bwd_tc_kernel(const __grid_con
                     mma_ts(tmem + DZ_COL + buf * 64, tmem + A_COL + (next ? 0 : 64) + 8 * jj, g_n + gs * SLOT + (uint64_t)(jj * 128), id_dz,
                            (next || jj) ? 1u : 0u);
             };
-            // all products of the 16-column K steps that hold the same channels: heads are steps 0, 1, remainders 2, 3
+            // all products of the 16-column K steps that hold the same channels: heads are steps 0, 1, remainders 2, 3; the
+            // products of heads last (the tensor core truncates an accumulator at every step, the small ones cost little)
             auto w_part = [&](uint32_t gs, uint32_t zs, uint32_t col, uint32_t idesc, bool first) {
 #pragma unroll
-                for (int m = 0; m < 8; ++m) {
+                for (int m = 7; m >= 0; --m) {
                     const int ka = (m & 1) + (m & 2), kb = (m & 1) + 2 * (m >> 2);
-                    mma_ss(tmem + W_COL + col, g_k + gs * SLOT + (uint64_t)(2 * ka), z_k + zs * SLOT + (uint64_t)(2 * kb), idesc,
-                           (first && m == 0) ? 0u : 1u);
+                    mma_ss(tmem + W_COL + col, g_k + gs * SLOT + (uint64_t)(2 * ka), z_k + zs * SLOT + (uint64_t)(2 * kb), idesc, (first && m == 7) ? 0u : 1u);
                 }
             };
-            uint32_t gc = 0, zc = 0, dc = 0;       // dc: dz accumulators begun
+            uint32_t gc = 0, zc = 0, dc = 0, wc = 0;       // dz accumulators and fillings of W begun
             bool ok = true;
             for (int t = 0; t < nmine && ok; ++t) {
                 if (!mbar_wait(bar(A_READY, 0), (uint32_t)(t & 1), 10)) break;
@@ -462,25 +413,39 @@ __global__ void __launch_bounds__(THREADS, 1) gcg_bwd_tc_kernel(const __grid_con
                     const uint32_t gs = gc % NG, zs = zc % NZ, zp = (zc - 1) % NZ;
                     if (!mbar_wait(bar(G_FULL, gs), (gc / NG) & 1u, 12)) { ok = false; break; }
                     tc_fence_after();
-                    if (k > 1) {
-                        dz_half(gs, (dc - 1) & 1u, true);
-                        mma_commit(bar(DZ_FULL, (dc - 1) & 1u));
+                    // W first if the last chunk's sums have left it: it is read while the dz halves run
+                    const bool early = mbar_test_wait(bar(Z_FULL, zs), (zc / NZ) & 1u) && (wc == 0 || (k - 1) % WCHUNKS || mbar_test_wait(bar(W_EMPTY, 0), (wc - 1) & 1u));
+#pragma unroll 1
+                    for (int part = 0; part < 2; ++part) {
+                        if ((part == 0) == early) {
+                            if (!mbar_wait(bar(Z_FULL, zs), (zc / NZ) & 1u, 13)) { ok = false; break; }
+                            const bool first = (k - 1) % WCHUNKS == 0;
+                            if (wc >= 1 && first && !mbar_wait(bar(W_EMPTY, 0), (wc - 1) & 1u, 16)) { ok = false; break; }
+                            tc_fence_after();
+                            if (zs == zp + 1) {            // the two z tiles are neighbours in the ring: 256 rows at once
+                                w_part(gs, zp, 0, id_w2, first);
+                            } else {
+                                w_part(gs, zp, 0, id_w1, first);
+                                w_part(gs, zs, 128, id_w1, first);
+                            }
+                            const bool last = k % WCHUNKS == 0 || k == n;
+                            if (last) mma_commit(bar(W_FULL, 0));
+                            mma_commit(bar(Z_FREE, zp));
+                            if (k == n) mma_commit(bar(Z_FREE, zs));
+                            wc += last;
+                        } else {
+                            if (k > 1) {
+                                dz_half(gs, (dc - 1) & 1u, true);
+                                mma_commit(bar(DZ_FULL, (dc - 1) & 1u));
+                            }
+                            // the accumulator was last read by the epilogue of the chunk before the previous one
+                            if (dc >= 2 && !mbar_wait(bar(DZ_EMPTY, dc & 1u), ((dc - 2) >> 1) & 1u, 14)) { ok = false; break; }
+                            tc_fence_after();
+                            dz_half(gs, dc & 1u, false);
+                        }
                     }
-                    // the accumulator was last read by the epilogue of the chunk before the previous one
-                    if (dc >= 2 && !mbar_wait(bar(DZ_EMPTY, dc & 1u), ((dc - 2) >> 1) & 1u, 14)) { ok = false; break; }
-                    tc_fence_after();
-                    dz_half(gs, dc & 1u, false);
-                    if (!mbar_wait(bar(Z_FULL, zs), (zc / NZ) & 1u, 13)) { ok = false; break; }
-                    tc_fence_after();
-                    if (zs == zp + 1) {            // the two z tiles are neighbours in the ring: 256 rows at once
-                        w_part(gs, zp, 0, id_w2, k == 1);
-                    } else {
-                        w_part(gs, zp, 0, id_w1, k == 1);
-                        w_part(gs, zs, 128, id_w1, k == 1);
-                    }
-                    mma_commit(bar(Z_FREE, zp));
+                    if (!ok) break;
                     mma_commit(bar(G_FREE, gs));
-                    if (k == n) mma_commit(bar(Z_FREE, zs));
                 }
                 if (!ok) break;
                 const uint32_t gs = gc % NG;
@@ -489,7 +454,6 @@ __global__ void __launch_bounds__(THREADS, 1) gcg_bwd_tc_kernel(const __grid_con
                 dz_half(gs, (dc - 1) & 1u, true);
                 mma_commit(bar(DZ_FULL, (dc - 1) & 1u));
                 mma_commit(bar(G_FREE, gs));
-                mma_commit(bar(W_FULL, 0));
                 ++gc;
             }
         }
@@ -532,6 +496,95 @@ __global__ void __launch_bounds__(THREADS, 1) gcg_bwd_tc_kernel(const __grid_con
                         ++gc;
                     }
                 }
+            }
+        }
+    } else {
+        // ======== dh: W out of TMEM after every other chunk, its anti-diagonals summed in fp32 registers over the item ============
+        const int e = warp % 4;                              // the lane quarter that this warp may read
+        const uint32_t lane_base = tmem + ((uint32_t)(e * 32) << 16);
+        // Anti-diagonals of W: row i (g2 at time 127 - i of the chunk) and column c (z at time c - 128 of it) meet at lag
+        // 255 - i - c, so a sum that moves one lane up per column to the left stays on its lag.  Columns from 255 - 32 e on
+        // leftwards hold the lags of this warp's rows, K + 31 of them those below K; four independent runs of a quarter of
+        // them hide the shuffle's latency.  Run q's lag rl q - 32 + p is complete in its word p: what has left lane 31 before
+        // its column p, or, from rl on, what lane rl + 31 - p holds at the end.  All go to shared memory (as vectors: shared
+        // memory and shuffles share a pipe that the tiles keep busy), and the sum over the runs is added to the lane's lags.
+        const int rl = (K + 31 + 8 * RUNS - 1) / (8 * RUNS) * 8;
+        const uint32_t sums = sm_u + OFF_RUNS + e * (RUNS * RUN_LAGS * 4);
+        auto read_w = [&](float (&dw)[CHUNK / 32]) {
+            float run[RUNS] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+            for (int c0 = 0; c0 < rl; c0 += 8) {
+                uint32_t w8[RUNS][8];
+#pragma unroll
+                for (int q = 0; q < RUNS; ++q) tmem_ld8(lane_base + W_COL + (uint32_t)(255 - 32 * e - rl * q - c0 - 7), w8[q]);
+                tmem_ld8_wait(w8[0], w8[1]);
+                tmem_ld8_wait(w8[2], w8[3]);
+                // the shuffle goes round: lane 0 gets what left lane 31, word c0 + j of the run
+                float left[RUNS][8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+#pragma unroll
+                    for (int q = 0; q < RUNS; ++q) {
+                        left[q][j] = __shfl_sync(0xffffffffu, run[q], lane + 31);
+                        run[q] = (lane ? left[q][j] : 0.f) + __uint_as_float(w8[q][7 - j]);
+                    }
+                if (lane == 0)
+#pragma unroll
+                    for (int q = 0; q < RUNS; ++q)
+#pragma unroll
+                        for (int j = 0; j < 8; j += 4)
+                            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(sums + (uint32_t)((q * RUN_LAGS + c0 + j) * 4)), "f"(left[q][j]),
+                                         "f"(left[q][j + 1]), "f"(left[q][j + 2]), "f"(left[q][j + 3]) : "memory");
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(W_EMPTY, 0));
+#pragma unroll
+            for (int q = 0; q < RUNS; ++q)
+                asm volatile("st.shared.f32 [%0], %1;" ::"r"(sums + (uint32_t)((q * RUN_LAGS + rl + 31 - lane) * 4)), "f"(run[q]) : "memory");
+            __syncwarp();
+#pragma unroll
+            for (int m = 0; m < CHUNK / 32; ++m) {
+                float v = 0.f;
+#pragma unroll
+                for (int q = 0; q < RUNS; ++q) {
+                    const int at = 32 * m + lane - rl * q + 32;
+                    if (at >= 1 && at < rl + 32) {
+                        float u;
+                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(u) : "r"(sums + (uint32_t)((q * RUN_LAGS + at) * 4)) : "memory");
+                        v += u;
+                    }
+                }
+                dw[m] += v;
+            }
+            __syncwarp();
+        };
+        uint32_t wc = 0;                      // fillings of W gone through
+        bool ok = true;
+        for (int t = 0; t < nmine && ok; ++t) {
+            const int g = item_group(t);
+            float dw[CHUNK / 32] = {};
+            for (int k = WCHUNKS; k < n + WCHUNKS; k += WCHUNKS, ++wc) {
+                if (!mbar_wait(bar(W_FULL, 0), wc & 1u, 8)) { ok = false; break; }
+                tc_fence_after();
+                __syncwarp();
+                read_w(dw);
+            }
+            if (!ok) break;
+            float* const dh = a.dh + (int64_t)((unsigned)(g * CH) / (unsigned)a.dg) * K;
+#pragma unroll
+            for (int m = 0; m < CHUNK / 32; ++m) {
+                const int lag = 32 * m + lane;
+                float v = dw[m];
+                if (__any_sync(0xffffffffu, lag < K && !isfinite(v))) {
+                    v = 0.f;
+#pragma unroll 1
+                    for (int s = 0; s < NS; ++s) {
+                        const Stream st = stream_of(a, item_set(t), s);
+                        if (st.active) v += dw_under_taps(a, st.b, (int64_t)g * CH, st.ts, st.te, CHUNK - 32 * (e + 1), lag);
+                    }
+                }
+                if (lag < K) atomicAdd(dh + (K - 1 - lag), v);
             }
         }
     }
