@@ -95,12 +95,6 @@ struct Args {
     int64_t hd;
 };
 
-__device__ __forceinline__ uint4 lds16(uint32_t addr) {      // (volatile: issued where it stands)
-    uint4 v;
-    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
-    return v;
-}
-
 template <bool INTERLEAVED, bool SWAP>
 __global__ void __launch_bounds__(THREADS, 1) fused_li_kernel(const __grid_constant__ CUtensorMap tmap, Args a) {
     extern __shared__ uint8_t smem_raw[];
