@@ -77,12 +77,10 @@ def launch_count() -> int:
 
 
 def _rows(B: int, R: int, L: int, like: torch.Tensor) -> torch.Tensor:
-    """Uninitialised [B, R, L] with every row on a 16-byte boundary: the first L samples of rows of whole 16-byte vectors
-    (a contiguous tensor where L is a multiple of them)."""
+    """Uninitialised [B, R, L] whose rows start on 16-byte boundaries (contiguous where L fills whole 16-byte vectors)."""
     n = 16 // like.element_size()
     pitch = -(-L // n) * n
-    t = torch.empty(B, R, pitch, device=like.device, dtype=like.dtype)
-    return t if pitch == L else t[..., :L]
+    return torch.empty_strided((B, R, L), (R * pitch, pitch, 1), device=like.device, dtype=like.dtype)
 
 
 # ----------------------------------------------------------------------------------------------
