@@ -122,6 +122,9 @@ int vtx_featurizer_fwd_pitched(const vtx_featurizer_params* p, int64_t z_pitch, 
  * of its batch row (two-level so that the per-head column split is a view).
  * round_kv != 0 rounds kv to the io dtype before the filter, as the
  * reference does when it materialises x1*v (engine.py:159).
+ * bf16 I/O and filters of up to 128 taps shared by blocks of 16 channels, on
+ * operand rows of 16-byte aligned starts, run on the tensor cores.  Infinite
+ * and NaN samples reach the outputs under the filter's taps and no others.
  * ------------------------------------------------------------------------ */
 typedef struct vtx_gcg_params {
     const void* q;  int64_t q_stride_b, q_stride_h, q_stride_d;
@@ -173,7 +176,8 @@ int vtx_gcg_cl_fwd_saving(const vtx_gcg_cl_params* p, void* y2, void* stream);
  * dx, dB, dC are contiguous [B,L,D] in the I/O dtype; dh32 is an fp32 [G,K] accumulator the caller zeroes (partial
  * sums are added with atomics: the order, hence the last bits, can differ between runs).  K <= 128; any I/O dtype;
  * fp32 accumulation: on the tensor cores for bf16 operands and filters shared by multiples of 16 channels (rows 16-byte
- * aligned, gradients 32-byte aligned), else on the CUDA cores. */
+ * aligned, gradients 32-byte aligned), else on the CUDA cores.  Infinite and NaN operands reach the gradients under the
+ * filter's taps and no others.  dh of random operands is about 3e-7 (CUDA cores: 5e-7) from its value in 64 bits. */
 typedef struct vtx_gcg_bwd_params {
     const void* dy;  int64_t dy_stride_b, dy_stride_l;
     const void* x;   int64_t x_stride_b, x_stride_l;

@@ -18,10 +18,12 @@
 // inner FIR cache from the last K-1 products of a sequence), 4-11 epilogue (thread = output sample, two warps per TMEM
 // lane quarter with two streams each: TMEM -> skip -> round -> gate, the result written over the q tile in place; the
 // first four also expand the next item's Toeplitz operand), 12 MMA issue, 13 TMA issue for k and v, 14 TMA issue for q,
-// 15 TMA stores of the finished tiles in whole 128-byte rows along time.  The epilogue is what bounds the kernel
+// 15 TMA stores of the finished tiles in whole 128-byte rows along time (the PLAIN form, for rows that no tensor map holds:
+// the epilogue stores its samples itself).  The epilogue is what bounds the kernel
 // (configuration B=4, L=8192, D=4096, 128 taps: 276 us with a round trip per channel pair, 251 with a stream's loads
-// together, 213 us = 0.77 of the HBM peak with the stores in a warp of their own; a third k*v slot: 222).  With fewer than
-// three batch elements the 32 boxes of a chunk are as many as the TMA unit retires (B=1, L=4001: 64 -> 51 us).  q
+// together, 213 us with the stores in a warp of their own; a third k*v slot: 222; 221 us = 0.74 of the HBM peak since sums that are not
+// finite are looked for and formed again).  With fewer than
+// three batch elements the 32 boxes of a chunk are as many as the TMA unit retires (B=1, L=4000: 55 us, L=4001 in the PLAIN form 61).  q
 // never passes through the front end: its tiles stay in their ring until their chunk's outputs have left through
 // them.  All waits are bounded.
 #include <cstdint>

@@ -87,8 +87,8 @@ def _rows(B: int, R: int, L: int, like: torch.Tensor) -> torch.Tensor:
 def featurizer_fwd(u_blc: torch.Tensor, w: torch.Tensor, bias=None, mask=None, want_state=True):
     """u_blc: logical [B, L, C] (any strides).  Returns z [B, C, L] and state [B, C, min(L,K-1)] or None.
 
-    Rows of z start on 16-byte boundaries, so z is a slice of a padded tensor when L is not a multiple of 16 bytes (as
-    the reference's fp32 z is a slice of the padded convolution, engine.py:197-204)."""
+    Rows of z start on 16-byte boundaries, so z is not dense when a row is no multiple of 16 bytes (as the reference's
+    fp32 z is a slice of the padded convolution, engine.py:197-204)."""
     _need_cuda(u_blc, w, bias, mask)
     B, L, Cc = u_blc.shape
     w = _param(w, u_blc).reshape(Cc, -1)
