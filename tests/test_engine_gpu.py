@@ -604,6 +604,48 @@ def test_long_conv_without_scratch(monkeypatch, B, L, D):
     check(f"long convolution without scratch L={L} state", rel_l2(st0, st), 2e-5)
 
 
+@pytest.mark.parametrize("L,K,masked", [(1, 3, False), (2, 3, True), (5, 8, False), (7, 3, False), (9, 8, True), (129, 4, False)])
+def test_featurizer_short_sequences(L, K, masked):
+    """Lengths below the filter's and below a vector on the kernel with tensor maps, which padded rows of z brought there:
+    the z and the cache of the general kernel (the same rows off the 16-byte boundaries), bit for bit."""
+    from vortex_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(L * K)
+    u = torch.randn(3, L, 72, device="cuda", generator=g).half()
+    w, b = torch.randn(72, 1, K, device="cuda", generator=g).half(), torch.randn(72, device="cuda", generator=g).half()
+    mask = (torch.rand(3, L, device="cuda", generator=g) > 0.3).half() if masked else None
+    off = torch.zeros(u.numel() + 1, device="cuda", dtype=u.dtype)[1:].view(u.shape).copy_(u)
+    for bias in (None, b):
+        for x, y in zip(ops.featurizer_fwd(u, w, bias, mask), ops.featurizer_fwd(off, w, bias, mask)):
+            assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("io,B,L,D", [("bf16", 2, 70, 40), ("f32", 1, 1001, 33)])
+def test_long_conv_channel_last_output(io, B, L, D):
+    """The C entry point with y strided as [B, L, D]: what it writes to [B, D, L], bit for bit."""
+    import ctypes as C
+
+    from vortex_b200 import _lib, ops
+
+    g = torch.Generator(device="cuda").manual_seed(L)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    z, bias, res = r(B, 3 * D, L).to(DT[io]), r(D).to(DT[io]), r(D, 16)
+    lp = torch.log(0.9 + 0.099 * torch.rand(D, 16, device="cuda", generator=g))
+    want, _ = ops.iir_fwd(z, lp, res, bias, D)
+    y = torch.full((B, L, D), float("nan"), device="cuda", dtype=z.dtype)
+    scratch = torch.empty(max(1, _lib.lib().vtx_iir_scratch_bytes(B, L, D, 16, 0)), device="cuda", dtype=torch.uint8)
+    code = {"bf16": _lib.BF16, "f32": _lib.F32}[io]
+    p = _lib.IirParams(head_dim=D, bias=bias.data_ptr(), bias_dtype=code, y=y.data_ptr(), y_stride_b=L * D, y_stride_d=1, y_stride_l=D,
+                       scratch=scratch.data_ptr(), B=B, L=L, D=D, round_kv=1, io_dtype=code)
+    for i, n in enumerate("qkv"):
+        setattr(p, n, z[:, i * D:].data_ptr())
+        setattr(p, n + "_stride_b", 3 * D * L)
+        setattr(p, n + "_stride_d", L)
+    p.modal = _lib.ModalParams(log_poles=lp.data_ptr(), res_re=res.data_ptr(), G=D, S=16)
+    _lib.check(_lib.lib().vtx_iir_fwd(C.byref(p), torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(y.transpose(1, 2), want)
+
+
 @pytest.mark.parametrize("L", [1000, 1003])       # the kernel with tensor maps takes both, z's rows being padded
 def test_featurizer_batch_pitches(L):
     """Batch pitches that no tensor map can hold: a single sequence whose (unused) pitch is odd, a batch expanded from one
