@@ -287,7 +287,8 @@ int vtx_iir_recurrence_fwd(const vtx_iir_params* p, void* stream);
  * free HBM to its cache pool, a C host without a device allocator, a latency-critical loop).  It has no
  * counterpart in the reference.  p->scratch is ignored: the segment carries live in an array of
  * VTX_IIR_STATIC_SCRATCH_BYTES that is part of the library image (each GPU that loads the library holds it
- * until exit).  Sizes needing more (see vtx_iir_scratch_bytes) return VTX_ERR_UNSUPPORTED.  The first call on
+ * until exit).  Sizes whose carries need more return VTX_ERR_UNSUPPORTED (none
+ * for which vtx_iir_scratch_bytes, an upper bound, answers no more than that).  The first call on
  * a device resolves the array's device address; make it before any stream capture.  With CUDA's default lazy
  * module loading the array's bytes are reserved on a device when the library's long-convolution module is first
  * used there (this first call, or the first vtx_iir_fwd / vtx_modal_filter), not when the library is loaded: make

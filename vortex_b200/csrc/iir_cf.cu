@@ -455,8 +455,8 @@ extern "C" int vtx_iir_recurrence_fwd(const vtx_iir_params* p, void* stream) {
 // library image, so every GPU that loads the library sets VTX_IIR_STATIC_SCRATCH_BYTES aside until the
 // process exits.  Inputs and outputs are still the caller's.
 //
-// * Sizes whose carries do not fit (vtx_iir_scratch_bytes(...) > VTX_IIR_STATIC_SCRATCH_BYTES) are refused
-//   with VTX_ERR_UNSUPPORTED; nothing is launched.  (What the launch's own plan needs always fits: at
+// * Sizes whose carries do not fit are refused with VTX_ERR_UNSUPPORTED (vtx_iir_scratch_bytes is an upper bound of
+//   them); nothing is launched.  (What the launch's own plan needs always fits: at
 //   most 148 * 16 * 32 carries of at most 16 complex states, 9.3 of the 16 MiB.)
 // * The first call on a device looks the array's device address up (cudaGetSymbolAddress with that device
 //   current -- the array's name is only a host-side handle, never a pointer a kernel could use) and keeps it
